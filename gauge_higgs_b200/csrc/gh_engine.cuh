@@ -38,7 +38,8 @@ struct Bufs {
   int gen_pair;    // 1: general-irrep link work through k_gen_pair (gen.w2_64 set)
   int gen_warps;   // warps per block of k_gen_links (1..GEN_WARPS, from the tensor size)
   int* blk_first;  // [nlat+1] first site item of each lattice (relative to the site items)
-  Work* w_kick;    // kick items over 4-D tiles (LatDev::lt): link items then site items
+  Work* w_kick;    // kick items: link items then site items, over 4-D tiles (LatDev::lt) or consecutive sites
+  int kick_lin;    // 1: some items are consecutive sites
   int nwk_links, nwk_sites;
   double* partials;
   double* res;
@@ -103,7 +104,8 @@ struct Engine : EngineBase {
     const int count = (links ? b.nwk_links : 0) + (do_sites ? b.nwk_sites : 0);
     if (count == 0) return;
     a.work = b.w_kick + first;
-    launch(k_kick<D, N, R, REP>, count, KICK_BLOCK, 0, b.st, a);
+    if (b.kick_lin) launch(k_kick<D, N, R, REP, true>, count, KICK_BLOCK, 0, b.st, a);
+    else launch(k_kick<D, N, R, REP, false>, count, KICK_BLOCK, 0, b.st, a);
   }
   void gen_links(const Bufs& b, double eps, int mode, double* out) override {
     if (REP != REP_GEN) return;

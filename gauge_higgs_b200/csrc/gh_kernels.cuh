@@ -64,6 +64,7 @@ struct LatDev {
   unsigned long long traj, accepted, nonfinite;
   int last_acc;
   int lt[4];                     // kick tile shape: log2 of the tile extent per direction
+  unsigned mag[4];               // floor(2^32 / L) (L = 1: 2^32 - 1): site_divmod's multiplier
   // Domain decomposition (src/mpi/gauge_mpi.hpp:26-80): a subdomain is stored with a
   // width-1 halo in every split direction.  Kernels act on the active box [lo, hi) only
   // (the whole lattice when not decomposed), and the counter RNG is keyed on the global
@@ -117,8 +118,10 @@ __device__ __forceinline__ long long global_site(const LatDev& L, int s) {
 }
 // Block work item.  Linear items: sites s0 .. s0+n-1.  Kick items (tiles): s0 is
 // the tile's origin site and n packs the origin coordinates, 8 bits each.
-// mu = -1 marks a site item, mu >= 0 a link item of direction mu.
+// mu = -1 marks a site item, mu >= 0 a link item of direction mu.  Linear kick items
+// carry mu + KICK_LINEAR.
 struct Work { int lat, mu, s0, n; };
+constexpr int KICK_LINEAR = 16;
 
 struct GenTables {                 // general irrep (src/rep/rep_general.hpp), sparse
   int d, n, dimT, ng;
@@ -206,10 +209,29 @@ __device__ __forceinline__ void st_link(R* U, const LatDev& L, int mu, int s, co
   for (int c = 0; c < N * N; ++c) stc<C>(U, base + c * ULANE, M.e[c]);
 }
 
+// (q, r) = (s / L, s % L) as a multiply-high and one correction: with mag = floor(2^32 / L)
+// the estimate s mag / 2^32 lies below s / L by s (2^32 / L - mag) / 2^32 < 1 for every
+// 32-bit s (L = 1: mag = 2^32 - 1, below by s / 2^32), so it is q or q - 1.
+__host__ __device__ __forceinline__ void site_divmod(unsigned s, unsigned L, unsigned mag, unsigned& q, unsigned& r) {
+#if defined(__CUDA_ARCH__)
+  q = __umulhi(s, mag);
+#else
+  q = (unsigned)(((unsigned long long)s * mag) >> 32);
+#endif
+  r = s - q * L;
+  if (r >= L) { r -= L; ++q; }
+}
+__host__ inline unsigned site_mag(int L) { return L == 1 ? 0xFFFFFFFFu : (unsigned)((1ULL << 32) / (unsigned)L); }
 template <int D> __device__ __forceinline__ void coords(const LatDev& L, int s, int* x) {
-  int r = s;
+  unsigned rest = (unsigned)s;
 #pragma unroll
-  for (int mu = 0; mu < D; ++mu) { x[mu] = r % L.L[mu]; r /= L.L[mu]; }
+  for (int mu = 0; mu < D; ++mu) {
+    if (mu == D - 1) { x[mu] = (int)rest; break; }
+    unsigned q, r;
+    site_divmod(rest, (unsigned)L.L[mu], L.mag[mu], q, r);
+    x[mu] = (int)r;
+    rest = q;
+  }
 }
 // neighbour of site s (whose coordinate in direction mu is xm) in +mu / -mu
 __device__ __forceinline__ int nfwd(const LatDev& L, int s, int xm, int mu) {
@@ -539,14 +561,26 @@ template <int REP> struct KickMinBlocks<double, REP> {
   static constexpr int v = b * 128 / KICK_BLOCK > 0 ? b * 128 / KICK_BLOCK : 1;
 };
 
-template <int D, int N, typename R, int REP>
+// LIN: the table holds linear items (and perhaps tiles); without, tiles only.  An instance
+// of its own: the FP32 kernel at 72 registers lost 1.7% at 16^4 with both forms inside.
+template <int D, int N, typename R, int REP, bool LIN>
 __global__ void __launch_bounds__(KICK_BLOCK, KickMinBlocks<R, REP>::v) k_kick(const KickArgs a) {
   pdl_enter();
   const Work w = a.work[blockIdx.x];
   const LatDev& L = a.lats[w.lat];
-  int s, x[D];
-  if (!tile_site<D>(L, w, threadIdx.x, s, x)) return;
-  if (w.mu >= 0) kick_link_dispatch<D, N, R, REP>(a, L, w.mu, s, x);
+  int s, x[D], mu = w.mu;
+  if (LIN && mu >= KICK_LINEAR - 1) {
+    // consecutive sites: extents that power-of-two tiles do not divide (rule and figures
+    // at kick_linear, gh_ctx.cu)
+    mu -= KICK_LINEAR;
+    if ((int)threadIdx.x >= w.n) return;
+    s = w.s0 + (int)threadIdx.x;
+    coords<D>(L, s, x);
+    if (L.dec && !in_box<D>(L, x)) return;
+  } else if (!tile_site<D>(L, w, threadIdx.x, s, x)) {
+    return;
+  }
+  if (mu >= 0) kick_link_dispatch<D, N, R, REP>(a, L, mu, s, x);
   else if (REP != REP_NONE) kick_site<D, N, R, REP>(a, L, s, x);
 }
 
