@@ -169,6 +169,50 @@ void eval(const Product& p, const double* U, double* Dout) {
   }
 }
 
+bool sym2_map(const Product& p, Sym2Map& out) {
+  if (p.K != 2) return false;
+  const int N = p.N, ng = N * N - 1, d = p.d, NN = N * N;
+  const std::vector<cd> T = ghpot::gell_mann(N);
+  // full tensors, index ((i N + j) N + k) N + l
+  std::vector<cd> F((size_t)NN * NN * d, cd(0.0, 0.0));
+  for (int a = 0; a < ng; ++a)
+    for (int b = 0; b < ng; ++b)
+      for (int i = 0; i < N; ++i)
+        for (int k = 0; k < N; ++k) {
+          const cd ta = 2.0 * T[(size_t)a * NN + i * N + k];
+          if (ta == cd(0.0, 0.0)) continue;
+          for (int j = 0; j < N; ++j)
+            for (int l = 0; l < N; ++l) {
+              const cd tab = ta * T[(size_t)b * NN + j * N + l];
+              if (tab == cd(0.0, 0.0)) continue;
+              const size_t e = ((size_t)(i * N + j) * N + k) * N + l;
+              for (int m = 0; m < d; ++m) F[e * d + m] += tab * p.Q[(size_t)(a * ng + b) * d + m];
+            }
+        }
+  double mx = 0.0;
+  for (const cd& z : F) mx = std::max(mx, std::abs(z));
+  const double tol = 1e-13 * mx;
+  out.NS = N * (N + 1) / 2;
+  out.nz.clear();
+  int I = 0;
+  for (int i = 0; i < N; ++i)
+    for (int j = i; j < N; ++j, ++I) {
+      int J = 0;
+      for (int k = 0; k < N; ++k)
+        for (int l = k; l < N; ++l, ++J)
+          for (int m = 0; m < d; ++m) {
+            const cd z = F[(((size_t)(i * N + j) * N + k) * N + l) * d + m];
+            const cd sw[3] = {F[(((size_t)(j * N + i) * N + k) * N + l) * d + m], F[(((size_t)(i * N + j) * N + l) * N + k) * d + m],
+                              F[(((size_t)(j * N + i) * N + l) * N + k) * d + m]};
+            for (const cd& y : sw)
+              if (std::abs(y - z) > tol) return false;
+            if (std::fabs(z.imag()) > tol) return false;
+            if (std::fabs(z.real()) > tol) out.nz.push_back({I * out.NS + J, m, z.real()});
+          }
+    }
+  return true;
+}
+
 bool build(int N, int n, int d, long dimT, const double* Win, Product& out, std::string* why) {
   auto no = [&](const char* m) { if (why) *why = m; return false; };
   if (N != 2 && N != 3) return no("product of adjoints is built for SU(2) and SU(3)");

@@ -44,6 +44,17 @@ struct Product {
 // N = 2 or 3; false (reason in *why) when the irrep is not reached that way.
 bool build(int N, int n, int d, long dimT, const double* W, Product& out, std::string* why);
 
+// The two-fold product as tensors Phi^{ij}_{kl} = 2 sum_ab Q_{ab,m} T^a_ik T^b_jl of component
+// m: when they are real and symmetric in (i, j) and in (k, l), the map from components to
+// the entries (i <= j, k <= l), row-major over the NS = N (N + 1) / 2 pairs each (the
+// factor 2 makes it an isometry under the full sum over i, j, k, l).
+struct Sym2Map {
+  int NS = 0;
+  struct Nz { int e, m; double v; };       // entry, component, value; ordered by entry
+  std::vector<Nz> nz;
+};
+bool sym2_map(const Product& p, Sym2Map& out);
+
 // Adjoint matrix of an SU(N) link (host): D[a][b] = 2 Re Tr(T^a U T^b U^dag).
 void adjoint_matrix(int N, const double* U, double* Dadj);
 

@@ -422,6 +422,34 @@ int rebuild_kick_table(gh_ctx* ctx) {
   return upload_kick_items(ctx, items, nl, ns);
 }
 
+// Lift and projection tables of k_gen_sym2; false where the irrep has no symmetric-tensor
+// form or (a basis supplied by the caller that mixes weights) too many nonzeros for them.
+bool sym2_tables(const ghadj::Product& p, Sym2Tab& t) {
+  ghadj::Sym2Map m;
+  if (!ghadj::sym2_map(p, m) || m.nz.size() > S2_NNZ || p.d > S2_DMAX || m.NS * m.NS > S2_PAIRS) return false;
+  const int N = p.N, NS = m.NS;
+  std::vector<double> w;
+  for (int i = 0; i < N; ++i)
+    for (int j = i; j < N; ++j) w.push_back(i == j ? 1.0 : 2.0);
+  std::memset(&t, 0, sizeof(t));
+  int n = 0;
+  for (int e = 0; e < NS * NS; ++e) {
+    for (const auto& z : m.nz)
+      if (z.e == e) { t.lm[n] = (unsigned char)z.m; t.lc64[n] = z.v; t.lc32[n] = (float)z.v; ++n; }
+    t.lptr[e + 1] = (unsigned char)n;
+  }
+  n = 0;
+  for (int k = 0; k < p.d; ++k) {
+    for (const auto& z : m.nz)
+      if (z.m == k) {
+        const double v = z.v * w[z.e / NS] * w[z.e % NS];
+        t.pe[n] = (unsigned char)z.e; t.pc64[n] = v; t.pc32[n] = (float)v; ++n;
+      }
+    t.pptr[k + 1] = (unsigned char)n;
+  }
+  return true;
+}
+
 int build_general(gh_ctx* ctx, const gh_rep_desc* r) {
   const int d = r->d, N = ctx->N, ng = ctx->ng;
   const long dimT = r->dimT;
@@ -482,7 +510,7 @@ int build_general(gh_ctx* ctx, const gh_rep_desc* r) {
   if (!t_v.empty()) CK(cudaMemcpyAsync(v3, t_v.data(), t_v.size() * 16, cudaMemcpyHostToDevice, ctx->st));
   t.wt_ptr = p1; t.wt_l = p2; t.wt_v = v1; t.w_ptr = p3; t.w_i = p4; t.w_v = v2; t.t_ptr = p5; t.t_j = p6; t.t_v = v3;
   t.sp_ptr = nullptr; t.sp_c = nullptr; t.sp_e = nullptr;
-  t.pq64 = nullptr; t.pq32 = nullptr; t.prow = nullptr; t.pK = 0; t.pnrows = 0; t.pndiag = 0; t.psym = 0;
+  t.pq64 = nullptr; t.pq32 = nullptr; t.prow = nullptr; t.pK = 0; t.pnrows = 0; t.pndiag = 0; t.psym = 0; t.s2 = 0;
   if (ctx->has_prod) {
     const std::vector<std::complex<double>>& Q = ctx->prod.Qr;
     std::vector<double2> q64(Q.size());
@@ -502,6 +530,7 @@ int build_general(gh_ctx* ctx, const gh_rep_desc* r) {
     CK(cudaStreamSynchronize(ctx->st));     // the host vectors go out of scope
     t.pq64 = d64; t.pq32 = d32; t.prow = rows; t.pK = ctx->prod.K;
     t.pnrows = (int)ctx->prod.rows.size(); t.pndiag = ctx->prod.ndiag; t.psym = ctx->prod.sym;
+    t.s2 = sym2_tables(ctx->prod, ctx->b.s2tab) ? 1 : 0;
   }
   t.w2_64 = nullptr; t.w2_32 = nullptr;
   if (ctx->has_pair) {

@@ -143,6 +143,7 @@ struct GenTables {                 // general irrep (src/rep/rep_general.hpp), s
   const double2* pq64; const float2* pq32;
   const int* prow;
   int pK, pnrows, pndiag, psym;
+  int s2;                          // 1: the two-fold product as symmetric tensors (k_gen_sym2; Bufs::s2tab)
   // two-slot irreps (n = 2): the basis W [d][N*N] dense in both precisions; null: not used
   const double2* w2_64; const float2* w2_32;
 };
@@ -1049,6 +1050,214 @@ __global__ void __launch_bounds__(GP_THREADS) k_gen_prod(const GenArgs a) {
       a.out[pi_] = (double)F;
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// Irreps of the two-fold adjoint product that are symmetric tensors: D_R(U) acts on
+//   Phi^{ij}_{kl} = 2 sum_ab (Q phi)_ab T^a_ik T^b_jl   as   U U Phi U^dag U^dag,
+// and when Phi is symmetric in (i, j) and in (k, l) (SU(3) 27-plet {4,2}, SU(2) {4}; the
+// host checks it, ghadj::sym2_map) its NS x NS entries, NS = N (N + 1) / 2, carry the irrep.
+// A column (fixed k <= l) is a symmetric N x N matrix M that becomes V M V^T with V = U,
+// a row (fixed i <= j) the same with V = conj(U), each by one thread with U in registers
+// (SU(3): 45 complex multiply-adds).  Lift and projection are real and sparse in this
+// basis (27-plet: 55 nonzeros of 36 x 27, where the intertwiner into the generators'
+// basis is dense: 2 x 972 complex multiply-adds per apply).  The matter force
+// g^a = -2 Im phi_x^dag T^a_R psi, with T^a_R acting on every index, is
+//   F = 4 kappa Im Tr T^a (A - B^T),  A = sum_J w_J M_psi M_x^dag, B = sum_I w_I N_psi N_x^dag
+// over columns J and rows I (w = 1 on the diagonal pairs, 2 off it).
+// Split: one block per 32 links of a direction, a warp per column (then per row), a lane
+// per link: shared memory is read without conflicts and every table entry is uniform.
+// Bound: latency, on 18 warps per SM (FP64 pipe 29% busy, shared memory 45%; about 7,000
+// multiply-adds per link).  3 blocks per SM (312 bytes spilled) beat 2 without spills by 4%,
+// FP32 5 beat 4 by 2%.
+// ---------------------------------------------------------------------------
+constexpr int S2_NNZ = 64, S2_DMAX = 36, S2_PAIRS = 36;   // largest tables the kernel takes
+struct Sym2Tab {
+  unsigned char lptr[S2_PAIRS + 4], lm[S2_NNZ];    // lift: rows IJ, components m
+  unsigned char pptr[S2_DMAX + 4], pe[S2_NNZ];     // projection: rows m, entries IJ
+  double lc64[S2_NNZ], pc64[S2_NNZ];               // pc: conj of the lift times w_I w_J
+  float lc32[S2_NNZ], pc32[S2_NNZ];
+};
+struct Sym2Args { GenArgs g; Sym2Tab t; };
+template <int N> struct Sym2 {
+  static constexpr int NS = N * (N + 1) / 2, THREADS = 32 * NS;
+  __host__ __device__ static constexpr int pair(int i, int j) { return i <= j ? i * N - i * (i - 1) / 2 + j - i : j * N - j * (j - 1) / 2 + i - j; }
+};
+// 32-lane complex rows of one phi buffer; the force's NS x ng real partial sums take its place later
+template <int N> __host__ __device__ constexpr int sym2_rows(int d) {
+  const int need = (Sym2<N>::NS * (N * N - 1) + 1) / 2;
+  return d > need ? d : need;
+}
+// phi_x, phi_{x+mu} (then the force's partial sums), the tensor
+template <int N, typename C> __host__ __device__ constexpr size_t sym2_smem(int d) {
+  return (size_t)(2 * sym2_rows<N>(d) + Sym2<N>::NS * Sym2<N>::NS) * 32 * 2 * sizeof(C);
+}
+// O = V M V^T for a symmetric M (pairs i <= j); V_ij = U_ij, transposed (TR) and / or conjugated (CJ)
+template <int N, bool TR, bool CJ, typename C>
+__device__ __forceinline__ void sym2_rotate(const Mat<N, C>& U, const cx<C>* M, cx<C>* O) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    cx<C> t[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      t[j] = zero<C>();
+#pragma unroll
+      for (int k = 0; k < N; ++k) {
+        const cx<C> v = U.e[TR ? k * N + i : i * N + k];
+        t[j] = CJ ? cfma_cj(t[j], v, M[Sym2<N>::pair(k, j)]) : cfma(t[j], v, M[Sym2<N>::pair(k, j)]);
+      }
+    }
+#pragma unroll
+    for (int j = i; j < N; ++j) {
+      cx<C> s = zero<C>();
+#pragma unroll
+      for (int k = 0; k < N; ++k) {
+        const cx<C> v = U.e[TR ? k * N + j : j * N + k];
+        s = CJ ? cfma_cj(s, v, t[k]) : cfma(s, v, t[k]);
+      }
+      O[Sym2<N>::pair(i, j)] = s;
+    }
+  }
+}
+// F += or -= w Im Tr T^a (P X^dag)  (or its transpose), P and X symmetric
+template <int N, bool MINUS_T, typename C>
+__device__ __forceinline__ void sym2_force(const cx<C>* P, const cx<C>* X, C w, C* F) {
+  Mat<N, C> R;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      cx<C> s = zero<C>();
+#pragma unroll
+      for (int k = 0; k < N; ++k) s = cfma_cj(s, X[Sym2<N>::pair(k, j)], P[Sym2<N>::pair(i, k)]);
+      R.e[MINUS_T ? j * N + i : i * N + j] = s;
+    }
+  C f[N * N - 1];
+  im_tr_proj<N, C>(R, f);
+#pragma unroll
+  for (int g = 0; g < N * N - 1; ++g) F[g] = fmad(MINUS_T ? -w : w, f[g], F[g]);
+}
+
+template <typename C> __device__ __forceinline__ C s2_lift(const Sym2Tab& t, int p) {
+  if constexpr (sizeof(C) == sizeof(double)) return t.lc64[p];
+  else return t.lc32[p];
+}
+template <typename C> __device__ __forceinline__ C s2_proj(const Sym2Tab& t, int p) {
+  if constexpr (sizeof(C) == sizeof(double)) return t.pc64[p];
+  else return t.pc32[p];
+}
+
+template <int D, int N, typename R>
+__global__ void __launch_bounds__(Sym2<N>::THREADS, sizeof(R) == 8 ? 3 : 5) k_gen_sym2(const __grid_constant__ Sym2Args a) {
+  pdl_enter();
+  typedef typename Cmp<R>::t C;
+  constexpr int NS = Sym2<N>::NS, ng = N * N - 1;
+  extern __shared__ unsigned char smem_raw[];
+  const Work w = a.g.work[blockIdx.x];
+  const LatDev& L = a.g.lats[w.lat];
+  const int d = a.g.t.d;
+  const int c = threadIdx.x & 31, q = threadIdx.x >> 5;   // lane: link; warp: column J, then row I
+  cx<C>* Px = reinterpret_cast<cx<C>*>(smem_raw) + c;     // [d][32] phi_x
+  cx<C>* Py = Px + 32 * sym2_rows<N>(d);                  // [d][32] phi_{x+mu}
+  cx<C>* X = Py + 32 * sym2_rows<N>(d);                   // [NS][NS][32]
+  C* Fs = reinterpret_cast<C*>(Py - c) + c;               // [NS][ng][32], once phi_{x+mu} is lifted
+  const int mu = w.mu;
+  const int s = w.s0 + (c < w.n ? c : 0);                 // lanes past the lattice's end compute on site s0
+  int x[D];
+  coords<D>(L, s, x);
+  const bool live = c < w.n && below_hi<D>(L, x);         // and store nothing, as upper halo sites of a subdomain
+  const bool own = live && in_box<D>(L, x);               // momentum updates: interior links only
+  const int spm = nfwd(L, s, x[mu], mu);
+  const R* phi = (const R*)a.g.phi;
+  for (int k = q; k < d; k += NS) {
+    Px[k * 32] = ldc<C>(phi, f_index(L, d, k, s));
+    Py[k * 32] = ldc<C>(phi, f_index(L, d, k, spm));
+  }
+  const Mat<N, C> U = ld_link<N, C>((const R*)a.g.U, L, mu, s);
+  auto lift = [&](const cx<C>* v, int e0, int step, cx<C>* M) {   // entries e0 + step i of the tensor of v
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+      M[i] = zero<C>();
+      const int e = e0 + step * i, p1 = a.t.lptr[e + 1];
+      for (int p = a.t.lptr[e]; p < p1; ++p) {
+        const cx<C> z = v[a.t.lm[p] * 32];
+        const C l = s2_lift<C>(a.t, p);
+        M[i].re = fmad(l, z.re, M[i].re);
+        M[i].im = fmad(l, z.im, M[i].im);
+      }
+    }
+  };
+  auto project = [&](R* out) {
+    for (int m = q; m < d; m += NS) {
+      cx<C> z = zero<C>();
+      const int p1 = a.t.pptr[m + 1];
+      for (int p = a.t.pptr[m]; p < p1; ++p) {
+        const cx<C> v = X[a.t.pe[p] * 32];
+        const C l = s2_proj<C>(a.t, p);
+        z.re = fmad(l, v.re, z.re);
+        z.im = fmad(l, v.im, z.im);
+      }
+      if (live) stc<C>(out, g_index(L, d, mu, m, s), z);
+    }
+  };
+  // w_q: 1 on the diagonal pairs, 2 off it
+  bool diag = false;
+#pragma unroll
+  for (int i = 0; i < N; ++i) diag = diag || q == Sym2<N>::pair(i, i);
+  const C k4 = C(4) * (C)L.kappa * (diag ? C(1) : C(2));
+  __syncthreads();
+  cx<C> M[NS], O[NS];
+  lift(Py, q, NS, M);                                     // psi_f = D phi_{x+mu}: columns, U
+  sym2_rotate<N, false, false, C>(U, M, O);
+#pragma unroll
+  for (int i = 0; i < NS; ++i) X[(i * NS + q) * 32] = O[i];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < NS; ++i) M[i] = X[(q * NS + i) * 32];   // rows, conj(U)
+  sym2_rotate<N, false, true, C>(U, M, O);
+#pragma unroll
+  for (int i = 0; i < NS; ++i) X[(q * NS + i) * 32] = O[i];
+  C F[ng];
+  if (a.g.mode != 1) {
+#pragma unroll
+    for (int g = 0; g < ng; ++g) F[g] = C(0);
+    lift(Px, q * NS, 1, M);
+    sym2_force<N, true, C>(O, M, k4, F);
+  }
+  __syncthreads();
+  project((R*)a.g.psif);
+  if (a.g.mode == 1) return;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) O[i] = X[(i * NS + q) * 32];
+  lift(Px, q, NS, M);
+  sym2_force<N, false, C>(O, M, k4, F);
+#pragma unroll
+  for (int g = 0; g < ng; ++g) Fs[(q * ng + g) * 32] = F[g];
+  __syncthreads();
+  if (own)
+    for (int g = q; g < ng; g += NS) {
+      double f = 0.0;
+#pragma unroll
+      for (int j = 0; j < NS; ++j) f += (double)Fs[(j * ng + g) * 32];
+      const long long pi_ = p_index(L, ng, mu, g, s);
+      if (a.g.mode == 0) {
+        R* P = (R*)a.g.P;
+        P[pi_] = (R)((C)P[pi_] - (C)a.g.eps * (C)f);
+      } else {
+        a.g.out[pi_] = f;
+      }
+    }
+  sym2_rotate<N, true, true, C>(U, M, O);                 // psi_b = D^dag phi_x: columns, U^dag
+#pragma unroll
+  for (int i = 0; i < NS; ++i) X[(i * NS + q) * 32] = O[i];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < NS; ++i) M[i] = X[(q * NS + i) * 32];   // rows, U^T
+  sym2_rotate<N, true, false, C>(U, M, O);
+#pragma unroll
+  for (int i = 0; i < NS; ++i) X[(q * NS + i) * 32] = O[i];
+  __syncthreads();
+  project((R*)a.g.psib);
 }
 
 // ---------------------------------------------------------------------------
