@@ -169,6 +169,19 @@ void eval(const Product& p, const double* U, double* Dout) {
   }
 }
 
+bool matrix_map(const Product& p, std::vector<cd>& W) {
+  if (p.K != 1) return false;
+  const int NN = p.N * p.N;
+  const std::vector<cd> T = ghpot::gell_mann(p.N);
+  W.assign((size_t)p.d * NN, cd(0.0, 0.0));
+  for (int m = 0; m < p.d; ++m)
+    for (int a = 0; a < NN - 1; ++a)
+      for (int t = 0; t < NN; ++t) W[(size_t)m * NN + t] += std::sqrt(2.0) * p.Q[(size_t)a * p.d + m] * T[(size_t)a * NN + t];
+  // entries that the weights rule out are rounding residue of the sums over a
+  for (cd& z : W) z = cd(std::fabs(z.real()) < 1e-15 ? 0.0 : z.real(), std::fabs(z.imag()) < 1e-15 ? 0.0 : z.imag());
+  return true;
+}
+
 bool sym2_map(const Product& p, Sym2Map& out) {
   if (p.K != 2) return false;
   const int N = p.N, ng = N * N - 1, d = p.d, NN = N * N;

@@ -55,6 +55,9 @@ struct Sym2Map {
 };
 bool sym2_map(const Product& p, Sym2Map& out);
 
+// The one-fold product as N x N matrices W_m = sqrt 2 sum_a Q_am T^a, [d][N*N] (an isometry).
+bool matrix_map(const Product& p, std::vector<std::complex<double>>& W);
+
 // Adjoint matrix of an SU(N) link (host): D[a][b] = 2 Re Tr(T^a U T^b U^dag).
 void adjoint_matrix(int N, const double* U, double* Dadj);
 

@@ -450,6 +450,26 @@ bool sym2_tables(const ghadj::Product& p, Sym2Tab& t) {
   return true;
 }
 
+// A complex table on the device in both precisions.
+int upload_table(gh_ctx* ctx, const std::vector<std::complex<double>>& v, const double2** p64, const float2** p32) {
+  std::vector<double2> a(v.size());
+  std::vector<float2> b(v.size());
+  for (size_t i = 0; i < v.size(); ++i) {
+    a[i] = make_double2(v[i].real(), v[i].imag());
+    b[i] = make_float2((float)v[i].real(), (float)v[i].imag());
+  }
+  double2* d64;
+  float2* d32;
+  int rc;
+  if ((rc = dalloc(ctx, &d64, a.size())) || (rc = dalloc(ctx, &d32, b.size()))) return rc;
+  CK(cudaMemcpyAsync(d64, a.data(), a.size() * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
+  CK(cudaMemcpyAsync(d32, b.data(), b.size() * sizeof(float2), cudaMemcpyHostToDevice, ctx->st));
+  CK(cudaStreamSynchronize(ctx->st));     // the host vectors go out of scope
+  *p64 = d64;
+  *p32 = d32;
+  return GH_OK;
+}
+
 int build_general(gh_ctx* ctx, const gh_rep_desc* r) {
   const int d = r->d, N = ctx->N, ng = ctx->ng;
   const long dimT = r->dimT;
@@ -510,44 +530,24 @@ int build_general(gh_ctx* ctx, const gh_rep_desc* r) {
   if (!t_v.empty()) CK(cudaMemcpyAsync(v3, t_v.data(), t_v.size() * 16, cudaMemcpyHostToDevice, ctx->st));
   t.wt_ptr = p1; t.wt_l = p2; t.wt_v = v1; t.w_ptr = p3; t.w_i = p4; t.w_v = v2; t.t_ptr = p5; t.t_j = p6; t.t_v = v3;
   t.sp_ptr = nullptr; t.sp_c = nullptr; t.sp_e = nullptr;
-  t.pq64 = nullptr; t.pq32 = nullptr; t.prow = nullptr; t.pK = 0; t.pnrows = 0; t.pndiag = 0; t.psym = 0; t.s2 = 0;
-  if (ctx->has_prod) {
-    const std::vector<std::complex<double>>& Q = ctx->prod.Qr;
-    std::vector<double2> q64(Q.size());
-    std::vector<float2> q32(Q.size());
-    for (size_t i = 0; i < Q.size(); ++i) {
-      q64[i] = make_double2(Q[i].real(), Q[i].imag());
-      q32[i] = make_float2((float)Q[i].real(), (float)Q[i].imag());
-    }
-    double2* d64;
-    float2* d32;
-    if ((rc = dalloc(ctx, &d64, q64.size())) || (rc = dalloc(ctx, &d32, q32.size()))) return rc;
-    CK(cudaMemcpyAsync(d64, q64.data(), q64.size() * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(d32, q32.data(), q32.size() * sizeof(float2), cudaMemcpyHostToDevice, ctx->st));
-    int* rows;
-    if ((rc = dalloc(ctx, &rows, ctx->prod.rows.size()))) return rc;
-    CK(cudaMemcpyAsync(rows, ctx->prod.rows.data(), ctx->prod.rows.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));     // the host vectors go out of scope
-    t.pq64 = d64; t.pq32 = d32; t.prow = rows; t.pK = ctx->prod.K;
-    t.pnrows = (int)ctx->prod.rows.size(); t.pndiag = ctx->prod.ndiag; t.psym = ctx->prod.sym;
+  t.pq64 = nullptr; t.pq32 = nullptr; t.prow = nullptr; t.pnrows = 0; t.pndiag = 0; t.psym = 0; t.s2 = 0;
+  // the N x N matrix map: the two-slot basis itself, or the one-fold adjoint product's
+  std::vector<std::complex<double>> Wm;
+  if (ctx->has_pair) Wm.assign(reinterpret_cast<const std::complex<double>*>(r->W), reinterpret_cast<const std::complex<double>*>(r->W) + (size_t)d * dimT);
+  else if (ctx->has_prod) ghadj::matrix_map(ctx->prod, Wm);
+  t.w2_64 = nullptr; t.w2_32 = nullptr; t.w2_real = 1;
+  if (!Wm.empty()) {
+    for (const std::complex<double>& z : Wm) t.w2_real = t.w2_real && z.imag() == 0.0;
+    if ((rc = upload_table(ctx, Wm, &t.w2_64, &t.w2_32))) return rc;
+  } else if (ctx->has_prod) {
     t.s2 = sym2_tables(ctx->prod, ctx->b.s2tab) ? 1 : 0;
   }
-  t.w2_64 = nullptr; t.w2_32 = nullptr;
-  if (ctx->has_pair) {
-    const size_t nw = (size_t)r->d * r->dimT;
-    std::vector<double2> w64(nw);
-    std::vector<float2> w32(nw);
-    for (size_t i = 0; i < nw; ++i) {
-      w64[i] = make_double2(r->W[2 * i], r->W[2 * i + 1]);
-      w32[i] = make_float2((float)r->W[2 * i], (float)r->W[2 * i + 1]);
-    }
-    double2* d64;
-    float2* d32;
-    if ((rc = dalloc(ctx, &d64, nw)) || (rc = dalloc(ctx, &d32, nw))) return rc;
-    CK(cudaMemcpyAsync(d64, w64.data(), nw * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(d32, w32.data(), nw * sizeof(float2), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));     // the host vectors go out of scope
-    t.w2_64 = d64; t.w2_32 = d32;
+  if (ctx->has_prod && Wm.empty() && !t.s2) {
+    int* rows;
+    if ((rc = upload_table(ctx, ctx->prod.Qr, &t.pq64, &t.pq32)) || (rc = dalloc(ctx, &rows, ctx->prod.rows.size()))) return rc;
+    CK(cudaMemcpyAsync(rows, ctx->prod.rows.data(), ctx->prod.rows.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
+    t.prow = rows;
+    t.pnrows = (int)ctx->prod.rows.size(); t.pndiag = ctx->prod.ndiag; t.psym = ctx->prod.sym;
   }
   t.warp_bytes = (int)ctx->gen_warp_bytes;
   t.px_off = (int)ctx->gen_px_off;

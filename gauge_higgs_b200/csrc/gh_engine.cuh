@@ -34,8 +34,8 @@ struct Bufs {
   int nw_gen;
   Work* w_gprod;   // general irrep, product of adjoints: items of up to 32 links (one 32-site block)
   int nw_gprod;
-  int gen_prod;    // 1: general-irrep link work through k_gen_prod (gen.pq64 set)
-  int gen_pair;    // 1: general-irrep link work through k_gen_pair (gen.w2_64 set)
+  int gen_prod;    // 1: general-irrep link work through the adjoint product (k_gen_pair, k_gen_sym2 or k_gen_prod)
+  int gen_pair;    // 1: general-irrep link work through k_gen_pair (two-slot irreps)
   int gen_warps;   // warps per block of k_gen_links (1..GEN_WARPS, from the tensor size)
   int* blk_first;  // [nlat+1] first site item of each lattice (relative to the site items)
   Work* w_kick;    // kick items: link items then site items, over 4-D tiles (LatDev::lt) or consecutive sites
@@ -85,12 +85,9 @@ struct Engine : EngineBase {
   int prepare(const Bufs& b) override {
     if (REP != REP_GEN) return 0;
     cudaError_t e = cudaFuncSetAttribute(k_gen_links<D, N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gen_smem(b));
-    if (e == cudaSuccess && b.gen.pq64) {
-      e = b.gen.pK == 1 ? cudaFuncSetAttribute(k_gen_prod<D, N, R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)gen_prod_smem<N, 1, C>(b.d, b.gen.pnrows))
-                        : cudaFuncSetAttribute(k_gen_prod<D, N, R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)gen_prod_smem<N, 2, C>(b.d, b.gen.pnrows));
-    }
+    if (e == cudaSuccess && b.gen.pq64)
+      e = cudaFuncSetAttribute(k_gen_prod<D, N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)gen_prod_smem<N, C>(b.d, b.gen.pnrows));
     if (e == cudaSuccess && b.gen.s2)
       e = cudaFuncSetAttribute(k_gen_sym2<D, N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sym2_smem<N, C>(b.d));
     return e == cudaSuccess ? 0 : -1;
@@ -116,12 +113,16 @@ struct Engine : EngineBase {
     a.work = b.w_gen; a.lats = b.lats; a.U = b.U; a.P = b.P; a.phi = b.phi; a.psif = b.psif; a.psib = b.psib;
     a.t = b.gen; a.eps = eps; a.mode = mode; a.out = out;
     a.pot = b.pot; a.sa = b.sa64; a.wpot = b.wpot;
-    if (b.gen_pair && b.gen.w2_64 && b.pot != POT_MULTI) {  // two-slot irreps in registers, one thread per link
+    const bool prod = b.gen_prod && b.pot != POT_MULTI, pair = b.gen_pair && b.pot != POT_MULTI;  // the potential's w is computed by k_gen_links
+    if (b.gen.w2_64 && (prod || pair)) {  // N x N matrices in registers, one thread per link
       a.work = b.w_all;
-      launch(k_gen_pair<D, N, R>, b.nw_links, KBLOCK, 0, b.st, a);
+      if (prod && b.gen.w2_real) launch(k_gen_pair<D, N, R, true, true>, b.nw_links, KBLOCK, 0, b.st, a);
+      else if (prod) launch(k_gen_pair<D, N, R, true, false>, b.nw_links, KBLOCK, 0, b.st, a);
+      else if (b.gen.w2_real) launch(k_gen_pair<D, N, R, false, true>, b.nw_links, KBLOCK, 0, b.st, a);
+      else launch(k_gen_pair<D, N, R, false, false>, b.nw_links, KBLOCK, 0, b.st, a);
       return;
     }
-    if (b.gen_prod && b.gen.pq64 && b.pot != POT_MULTI) {   // the potential's w is computed by k_gen_links
+    if (prod && (b.gen.s2 || b.gen.pq64)) {
       a.work = b.w_gprod;
       // symmetric tensors wherever the irrep has them (27-plet, SU(2) {4}): SU(3) 27-plet
       // 12^4 FP64, cold caches, 112 us against k_gen_prod's 581
@@ -129,10 +130,9 @@ struct Engine : EngineBase {
         Sym2Args sa;
         sa.g = a; sa.t = b.s2tab;
         launch(k_gen_sym2<D, N, R>, b.nw_gprod, Sym2<N>::THREADS, sym2_smem<N, C>(b.d), b.st, sa);
-        return;
+      } else {
+        launch(k_gen_prod<D, N, R>, b.nw_gprod, GP_THREADS, gen_prod_smem<N, C>(b.d, b.gen.pnrows), b.st, a);
       }
-      if (b.gen.pK == 1) launch(k_gen_prod<D, N, R, 1>, b.nw_gprod, GP_THREADS, gen_prod_smem<N, 1, C>(b.d, b.gen.pnrows), b.st, a);
-      else launch(k_gen_prod<D, N, R, 2>, b.nw_gprod, GP_THREADS, gen_prod_smem<N, 2, C>(b.d, b.gen.pnrows), b.st, a);
       return;
     }
     const size_t sm = gen_smem(b);

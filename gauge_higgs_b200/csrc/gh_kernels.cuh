@@ -17,6 +17,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 #include "gh_math.cuh"
 #include "gh_rng.cuh"
 
@@ -142,10 +143,12 @@ struct GenTables {                 // general irrep (src/rep/rep_general.hpp), s
   // matrix the pairs a <= b / a < b): prow[r] = a ng + b, the first pndiag diagonal
   const double2* pq64; const float2* pq32;
   const int* prow;
-  int pK, pnrows, pndiag, psym;
+  int pnrows, pndiag, psym;
   int s2;                          // 1: the two-fold product as symmetric tensors (k_gen_sym2; Bufs::s2tab)
-  // two-slot irreps (n = 2): the basis W [d][N*N] dense in both precisions; null: not used
+  // irreps that are N x N matrices (two slots, or the one-fold adjoint product): the map
+  // W [d][N*N] dense in both precisions, and whether it is real; null: not used
   const double2* w2_64; const float2* w2_32;
+  int w2_real;
 };
 
 template <typename R> struct V2;
@@ -851,10 +854,10 @@ __global__ void __launch_bounds__(GEN_WARPS * 32) k_gen_links(const GenArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// General irreps inside the K-fold adjoint product (K = 1, 2; host set-up and the
-// algebra in gh_adjprod.h): with the fixed isometric intertwiner Q (A x d,
-// A = (N^2 - 1)^K) from the reference's basis into the product,
-//   D_R(U) phi = Q^dag (G (x) ... (x) G) Q phi,   G_ab = 2 Re Tr(T^a U T^b U^dag),
+// General irreps inside the two-fold adjoint product that are no symmetric tensors (10bar
+// {3,3}; host set-up and the algebra in gh_adjprod.h): with the fixed isometric
+// intertwiner Q (A x d, A = (N^2 - 1)^2) from the reference's basis into the product,
+//   D_R(U) phi = Q^dag (G (x) G) Q phi,   G_ab = 2 Re Tr(T^a U T^b U^dag),
 // and D_R(U)^dag phi with G^T.  One block takes the 32 links of one 32-site block and
 // one direction, 8 threads per link: the lift Q phi and the projection Q^dag y are
 // 64 x 27 and 27 x 64 products shared by the 32 links (every warp reads the same Q
@@ -866,23 +869,23 @@ __global__ void __launch_bounds__(GEN_WARPS * 32) k_gen_links(const GenArgs a) {
 // ---------------------------------------------------------------------------
 constexpr int GP_LINKS = 32;      // links per block (one 32-site block, one direction)
 constexpr int GP_THREADS = 256;   // 8 per link
-template <int N, int K> struct AdjProd {
+template <int N> struct AdjProd {
   static constexpr int NG = N * N - 1;
-  static constexpr int A = (K == 1) ? NG : NG * NG;
+  static constexpr int A = NG * NG;
   static constexpr int RA = (A + 7) / 8;      // rows of A (and of d <= A) per thread
 };
-template <int N, int K, typename C> __host__ __device__ constexpr size_t gen_prod_smem(int d, int nrows) {
-  return (size_t)nrows * d * sizeof(cx<C>) + (size_t)(2 * d + AdjProd<N, K>::A) * GP_LINKS * sizeof(cx<C>) +
-         (size_t)AdjProd<N, K>::NG * AdjProd<N, K>::NG * GP_LINKS * sizeof(C);
+template <int N, typename C> __host__ __device__ constexpr size_t gen_prod_smem(int d, int nrows) {
+  return (size_t)nrows * d * sizeof(cx<C>) + (size_t)(2 * d + AdjProd<N>::A) * GP_LINKS * sizeof(cx<C>) +
+         (size_t)AdjProd<N>::NG * AdjProd<N>::NG * GP_LINKS * sizeof(C);
 }
 
 // out[i] = (D phi)_k, k = q + 8 i, for the link in lane c; Pin: [d][32] input vectors;
 // Qs: [nrows][d] the rows of Q in shared memory; X: [A][32] work space; G: [NG][NG][32]
 // adjoint matrices.  Every thread of the block calls it.
-template <int N, int K, typename C>
+template <int N, typename C>
 __device__ __forceinline__ void gp_apply(const GenTables& t, const cx<C>* Qs, int d, const cx<C>* Pin, cx<C>* X,
                                          const C* G, bool dag, int c, int q, cx<C>* out) {
-  constexpr int NG = AdjProd<N, K>::NG, A = AdjProd<N, K>::A, RA = AdjProd<N, K>::RA, LB = GP_LINKS;
+  constexpr int NG = AdjProd<N>::NG, RA = AdjProd<N>::RA, LB = GP_LINKS;
   const int nr = t.pnrows;
   cx<C> acc[RA];
 #pragma unroll
@@ -896,14 +899,14 @@ __device__ __forceinline__ void gp_apply(const GenTables& t, const cx<C>* Qs, in
     }
   }
   __syncthreads();                                      // earlier readers of X are done
-  if (K == 2 && t.psym < 0 && q < NG) X[(q * NG + q) * LB + c] = zero<C>();   // antisymmetric: zero diagonal
+  if (t.psym < 0 && q < NG) X[(q * NG + q) * LB + c] = zero<C>();   // antisymmetric: zero diagonal
 #pragma unroll
   for (int i = 0; i < RA; ++i) {
     const int r = q + 8 * i;
     if (r < nr) {
       const int e = __ldg(t.prow + r);
       X[e * LB + c] = acc[i];
-      if (K == 2 && t.psym != 0) {
+      if (t.psym != 0) {
         const int a = e / NG, b = e - a * NG;
         if (a != b) X[(b * NG + a) * LB + c] = t.psym > 0 ? acc[i] : mk<C>(-acc[i].re, -acc[i].im);
       }
@@ -911,15 +914,7 @@ __device__ __forceinline__ void gp_apply(const GenTables& t, const cx<C>* Qs, in
   }
   __syncthreads();
   auto g = [&](int a, int b) { return dag ? G[(b * NG + a) * LB + c] : G[(a * NG + b) * LB + c]; };
-  if constexpr (K == 1) {                               // y = G x
-    cx<C> y = zero<C>();
-    const int a = q;
-    if (a < NG)
-#pragma unroll
-      for (int k = 0; k < NG; ++k) y = add(y, scale(X[k * LB + c], g(a, k)));
-    __syncthreads();
-    if (a < NG) X[a * LB + c] = y;
-  } else {                                              // Y = G X G^T, row a of this thread
+  {                                                     // Y = G X G^T, row a of this thread
     const int a = q;
     cx<C> y[NG];
     if (a < NG) {
@@ -959,11 +954,11 @@ __device__ __forceinline__ void gp_apply(const GenTables& t, const cx<C>* Qs, in
   }
 }
 
-template <int D, int N, typename R, int K>
+template <int D, int N, typename R>
 __global__ void __launch_bounds__(GP_THREADS) k_gen_prod(const GenArgs a) {
   pdl_enter();
   typedef typename Cmp<R>::t C;
-  constexpr int NG = AdjProd<N, K>::NG, A = AdjProd<N, K>::A, RA = AdjProd<N, K>::RA, LB = GP_LINKS;
+  constexpr int NG = AdjProd<N>::NG, A = AdjProd<N>::A, RA = AdjProd<N>::RA, LB = GP_LINKS;
   extern __shared__ unsigned char smem_raw[];
   const Work w = a.work[blockIdx.x];
   const LatDev& L = a.lats[w.lat];
@@ -1011,7 +1006,7 @@ __global__ void __launch_bounds__(GP_THREADS) k_gen_prod(const GenArgs a) {
   R* psif = (R*)a.psif;
   R* psib = (R*)a.psib;
   cx<C> o[RA];
-  gp_apply<N, K, C>(a.t, Qs, d, Py, X, G, false, c, q, o);  // psi_f = D phi_{x+mu}
+  gp_apply<N, C>(a.t, Qs, d, Py, X, G, false, c, q, o);  // psi_f = D phi_{x+mu}
 #pragma unroll
   for (int i = 0; i < RA; ++i) {
     const int k = q + 8 * i;
@@ -1021,7 +1016,7 @@ __global__ void __launch_bounds__(GP_THREADS) k_gen_prod(const GenArgs a) {
     }
   }
   if (a.mode == 1) return;
-  gp_apply<N, K, C>(a.t, Qs, d, Px, X, G, true, c, q, o);   // psi_b = D^dag phi_x
+  gp_apply<N, C>(a.t, Qs, d, Px, X, G, true, c, q, o);   // psi_b = D^dag phi_x
 #pragma unroll
   for (int i = 0; i < RA; ++i) {
     const int k = q + 8 * i;
@@ -1261,21 +1256,30 @@ __global__ void __launch_bounds__(Sym2<N>::THREADS, sizeof(R) == 8 ? 3 : 5) k_ge
 }
 
 // ---------------------------------------------------------------------------
-// Two-slot irreps (n = 2: the symmetric and antisymmetric squares of V, e.g. the SU(3)
-// sextet {2} and antitriplet {1,1}) in registers, one thread per link.  With the irrep
-// basis W ([d][N*N], tensor index i*N + j for the slots (i, j)) the reference's tensor
-// apply (src/rep/rep_general.hpp:184-220: lift with W, U on each slot, project with W^H)
-// is, as N x N matrices,
-//   Phi = sum_b phi_b W_b,  Psi = U Phi U^T,  psi_b = sum_ij conj(W_b,ij) Psi_ij,
-// and D^dag phi the same with Psi = U^dag Phi conj(U).  Every W_b is symmetric or
-// antisymmetric, so phi_x^dag T^a_R psi_f = Tr(Phi_x^dag (T^a Psi + Psi T^aT))
-// = 2 Tr(T^a Psi Phi_x^dag), and the matter force -kappa g^a, g^a = -2 Im(phi_x^dag
-// T^a_R D phi_{x+mu}) (src/rep/representation.hpp:36-46), is 4 kappa Im Tr(T^a Psi
-// Phi_x^dag): one N x N product and the projection the fundamental uses.  Outputs and
-// modes as k_gen_links: psi_f, psi_b to the scratch fields; mode 0 P -= eps F, mode 2
-// F -> out, mode 1 psi_f only.
+// Irreps that are N x N matrices, in registers, one thread per link.  With the map
+// Phi = sum_b phi_b W_b of d components to N x N matrices (an isometry, d x N^2 entries):
+//  ADJ false, two-slot irreps (n = 2: the symmetric and antisymmetric squares of V, e.g.
+//   the SU(3) sextet {2} and antitriplet {1,1}), W the irrep basis with tensor index
+//   i*N + j for the slots (i, j); the reference's tensor apply
+//   (src/rep/rep_general.hpp:184-220: lift with W, U on each slot, project with W^H) is
+//   Psi = U Phi U^T, and D^dag phi the same with U^dag Phi conj(U).  Every W_b is symmetric
+//   or antisymmetric, so phi_x^dag T^a_R psi_f = Tr(Phi_x^dag (T^a Psi + Psi T^aT))
+//   = 2 Tr(T^a Psi Phi_x^dag), and the matter force -kappa g^a, g^a = -2 Im(phi_x^dag
+//   T^a_R D phi_{x+mu}) (src/rep/representation.hpp:36-46), is 4 kappa Im Tr(T^a Psi
+//   Phi_x^dag): one N x N product and the projection the fundamental uses.
+//  ADJ true, the one-fold adjoint product (SU(3) octet {2,1}, SU(2) {2}), W_b = sqrt 2
+//   sum_a Q_ab T^a of the intertwiner Q: Psi = U Phi U^dag, D^dag the same with U^dag, and
+//   T^a_R psi the commutator [T^a, Psi], so the force is 2 kappa Im Tr T^a (Psi Phi_x^dag
+//   - Phi_x^dag Psi).
+// RW: W is real (every basis that gh_rep_general_build makes), a multiply-add per part.
+// psi_b then psi_f components leave by coalesced stores; modes and outputs as k_gen_links.
+// Bound: FP pipe and the latency of one link's chain of products.  ADJ against the 8 x 8
+// adjoint matrices in shared memory that it replaced (k_gen_prod), SU(3) octet 12^4 FP32:
+// kick with it 62.4 -> 25.4 us (FP64 98.0 -> 35.8); RW on the sextet: FP64 kick 42.1 -> 31.9 us
+// together with consecutive-site kick blocks.  5 FP32 blocks per SM (72 bytes spilled by the
+// octet): 12^4 has 4.4 blocks per SM, and 4 resident took 29.1 us.
 // ---------------------------------------------------------------------------
-template <int N, typename C, typename R>
+template <int N, bool RW, typename C, typename R>
 __device__ __forceinline__ Mat<N, C> pair_lift(const typename V2<C>::t* Wt, int d, const R* phi, const LatDev& L, int s) {
   Mat<N, C> M;
   set_zero(M);
@@ -1284,12 +1288,17 @@ __device__ __forceinline__ Mat<N, C> pair_lift(const typename V2<C>::t* Wt, int 
 #pragma unroll
     for (int t = 0; t < N * N; ++t) {
       const typename V2<C>::t v = __ldg(Wt + b * N * N + t);
-      M.e[t] = cfma(M.e[t], f, mk<C>(v.x, v.y));
+      if (RW) {
+        M.e[t].re = fmad(f.re, v.x, M.e[t].re);
+        M.e[t].im = fmad(f.im, v.x, M.e[t].im);
+      } else {
+        M.e[t] = cfma(M.e[t], f, mk<C>(v.x, v.y));
+      }
     }
   }
   return M;
 }
-template <int N, typename C, typename R>
+template <int N, bool RW, typename C, typename R>
 __device__ __forceinline__ void pair_project(const typename V2<C>::t* Wt, int d, const Mat<N, C>& M, R* out,
                                              const LatDev& L, int mu, int s) {
   for (int b = 0; b < d; ++b) {
@@ -1297,7 +1306,12 @@ __device__ __forceinline__ void pair_project(const typename V2<C>::t* Wt, int d,
 #pragma unroll
     for (int t = 0; t < N * N; ++t) {
       const typename V2<C>::t v = __ldg(Wt + b * N * N + t);
-      z = cfma(z, mk<C>(v.x, -v.y), M.e[t]);
+      if (RW) {
+        z.re = fmad(M.e[t].re, v.x, z.re);
+        z.im = fmad(M.e[t].im, v.x, z.im);
+      } else {
+        z = cfma(z, mk<C>(v.x, -v.y), M.e[t]);
+      }
     }
     stc<C>(out, g_index(L, d, mu, b, s), z);
   }
@@ -1308,8 +1322,8 @@ template <int N, typename C> __device__ __forceinline__ Mat<N, C> conj_mat(const
   for (int i = 0; i < N * N; ++i) B.e[i] = conj(A.e[i]);
   return B;
 }
-template <int D, int N, typename R>
-__global__ void __launch_bounds__(KBLOCK) k_gen_pair(const GenArgs a) {
+template <int D, int N, typename R, bool ADJ, bool RW>
+__global__ void __launch_bounds__(KBLOCK, sizeof(R) == 8 ? 3 : 5) k_gen_pair(const GenArgs a) {
   pdl_enter();
   typedef typename Cmp<R>::t C;
   const Work w = a.work[blockIdx.x];
@@ -1324,29 +1338,41 @@ __global__ void __launch_bounds__(KBLOCK) k_gen_pair(const GenArgs a) {
       sizeof(C) == sizeof(double) ? (const void*)a.t.w2_64 : (const void*)a.t.w2_32);
   const R* phi = (const R*)a.phi;
   const Mat<N, C> U = ld_link<N, C>((const R*)a.U, L, mu, s);
-  const Mat<N, C> Uc = conj_mat(U);
   const int spm = nfwd(L, s, x[mu], mu);
-  // psi_f = D phi_{x+mu}: U Phi U^T = (U Phi) conj(U)^dag
-  const Mat<N, C> Psi = mm_nd(mm(U, pair_lift<N, C>(Wt, d, phi, L, spm)), Uc);
-  pair_project<N, C>(Wt, d, Psi, (R*)a.psif, L, mu, s);
+  // psi_f = D phi_{x+mu}: U Phi U^T = (U Phi) conj(U)^dag, or U Phi U^dag
+  const Mat<N, C> Psi = mm_nd(mm(U, pair_lift<N, RW, C>(Wt, d, phi, L, spm)), ADJ ? U : conj_mat(U));
+  pair_project<N, RW, C>(Wt, d, Psi, (R*)a.psif, L, mu, s);
   if (a.mode == 1) return;
-  const Mat<N, C> Phx = pair_lift<N, C>(Wt, d, phi, L, s);
-  // psi_b = D^dag phi_x: U^dag Phi conj(U)
-  pair_project<N, C>(Wt, d, mm(mm_dn(U, Phx), Uc), (R*)a.psib, L, mu, s);
+  const Mat<N, C> Phx = pair_lift<N, RW, C>(Wt, d, phi, L, s);
+  // psi_b = D^dag phi_x: U^dag Phi conj(U), or U^dag Phi U
+  pair_project<N, RW, C>(Wt, d, mm(mm_dn(U, Phx), ADJ ? U : conj_mat(U)), (R*)a.psib, L, mu, s);
   if (!in_box<D>(L, x)) return;                        // momentum updates: interior links only
-  Mat<N, C> M = mm_nd(Psi, Phx);
-  const C k4 = C(4) * (C)L.kappa;
-#pragma unroll
-  for (int i = 0; i < N * N; ++i) M.e[i] = scale(M.e[i], k4);
+  // the commutator's terms cancel in part: in double, whatever the fields (FP32 octet force
+  // against FP64: 6.99e-8 rms with it, 9.34e-8 in FP32, 9.06e-8 in k_gen_prod's double sums)
+  typedef typename std::conditional<ADJ, double, C>::type S;
   constexpr int ng = N * N - 1;
-  C F[ng];
-  im_tr_proj<N, C>(M, F);
+  S F[ng];
+  {
+    Mat<N, S> Ps, Px;
+#pragma unroll
+    for (int i = 0; i < N * N; ++i) { Ps.e[i] = cvt<S>(Psi.e[i]); Px.e[i] = cvt<S>(Phx.e[i]); }
+    Mat<N, S> M = mm_nd(Ps, Px);
+    if (ADJ) {
+      const Mat<N, S> M2 = mm_dn(Px, Ps);
+#pragma unroll
+      for (int i = 0; i < N * N; ++i) M.e[i] = sub(M.e[i], M2.e[i]);
+    }
+    const S kf = S(ADJ ? 2 : 4) * (S)L.kappa;
+#pragma unroll
+    for (int i = 0; i < N * N; ++i) M.e[i] = scale(M.e[i], kf);
+    im_tr_proj<N, S>(M, F);
+  }
   const long long pb = p_index(L, ng, mu, 0, s);
   if (a.mode == 0) {
     R* P = (R*)a.P;
     const C eps = (C)a.eps;
 #pragma unroll
-    for (int g = 0; g < ng; ++g) P[pb + g * ULANE] = (R)((C)P[pb + g * ULANE] - eps * F[g]);
+    for (int g = 0; g < ng; ++g) P[pb + g * ULANE] = (R)((C)P[pb + g * ULANE] - eps * (C)F[g]);
   } else {
 #pragma unroll
     for (int g = 0; g < ng; ++g) a.out[pb + g * ULANE] = (double)F[g];
