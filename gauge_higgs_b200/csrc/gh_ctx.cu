@@ -355,11 +355,14 @@ void kick_items(const gh_ctx* ctx, const std::vector<int>& lats, std::vector<Wor
   const int D = ctx->D;
   for (int l : lats) {
     const LatDev& Ld = ctx->lat_h[l];
+    const bool split = ctx->rep == REP_GEN && ctx->d >= KICK_SITE_SPLIT_D;
+    if (split)
+      for (int s0 = 0; s0 < Ld.V; s0 += ULANE) sites.push_back(Work{l, -1, s0, std::min(ULANE, Ld.V - s0)});
     if (ctx->kick_lin[l]) {
       for (int s0 = 0; s0 < Ld.V; s0 += KICK_BLOCK) {
         const int n = std::min(KICK_BLOCK, Ld.V - s0);
         for (int mu = 0; mu < D; ++mu) links_mu[mu].push_back(Work{l, mu + KICK_LINEAR, s0, n});
-        sites.push_back(Work{l, KICK_LINEAR - 1, s0, n});
+        if (!split) sites.push_back(Work{l, KICK_LINEAR - 1, s0, n});
       }
       continue;
     }
@@ -376,7 +379,7 @@ void kick_items(const gh_ctx* ctx, const std::vector<int>& lats, std::vector<Wor
         packed |= o << (8 * mu);
       }
       for (int mu = 0; mu < D; ++mu) links_mu[mu].push_back(Work{l, mu, s0, packed});
-      sites.push_back(Work{l, -1, s0, packed});
+      if (!split) sites.push_back(Work{l, -1, s0, packed});
     }
   }
   for (int mu = 0; mu < D; ++mu) links.insert(links.end(), links_mu[mu].begin(), links_mu[mu].end());

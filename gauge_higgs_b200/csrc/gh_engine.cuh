@@ -104,8 +104,15 @@ struct Engine : EngineBase {
     const int count = (links ? b.nwk_links : 0) + (do_sites ? b.nwk_sites : 0);
     if (count == 0) return;
     a.work = b.w_kick + first;
-    if (b.kick_lin) launch(k_kick<D, N, R, REP, true>, count, KICK_BLOCK, 0, b.st, a);
-    else launch(k_kick<D, N, R, REP, false>, count, KICK_BLOCK, 0, b.st, a);
+    if constexpr (REP == REP_GEN) {
+      if (b.d >= KICK_SITE_SPLIT_D) {
+        if (b.kick_lin) launch(k_kick<D, N, R, REP, true, true>, count, KICK_BLOCK, 0, b.st, a);
+        else launch(k_kick<D, N, R, REP, false, true>, count, KICK_BLOCK, 0, b.st, a);
+        return;
+      }
+    }
+    if (b.kick_lin) launch(k_kick<D, N, R, REP, true, false>, count, KICK_BLOCK, 0, b.st, a);
+    else launch(k_kick<D, N, R, REP, false, false>, count, KICK_BLOCK, 0, b.st, a);
   }
   void gen_links(const Bufs& b, double eps, int mode, double* out) override {
     if (REP != REP_GEN) return;

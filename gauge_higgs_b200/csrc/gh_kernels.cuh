@@ -120,8 +120,9 @@ __device__ __forceinline__ long long global_site(const LatDev& L, int s) {
 // Block work item.  Linear items: sites s0 .. s0+n-1.  Kick items (tiles): s0 is
 // the tile's origin site and n packs the origin coordinates, 8 bits each.
 // mu = -1 marks a site item, mu >= 0 a link item of direction mu.  Linear kick items
-// carry mu + KICK_LINEAR.
+// carry mu + KICK_LINEAR, except kick_site_gen's (mu = -1), which hold up to 32 sites.
 struct Work { int lat, mu, s0, n; };
+constexpr int KICK_SITE_SPLIT_D = 9;   // components from which on kick_site_gen is used
 constexpr int KICK_LINEAR = 16;
 
 struct GenTables {                 // general irrep (src/rep/rep_general.hpp), sparse
@@ -513,7 +514,6 @@ __device__ __forceinline__ void kick_site(const KickArgs& a, const LatDev& L, in
       }
 #pragma unroll
       for (int mu = 0; mu < D; ++mu) {
-        
         F = add(F, scale(add(ldc<C>(psif, g_index(L, d, mu, k, s)), ldc<C>(psib, g_index(L, d, mu, k, yb[mu]))), kap2));
       }
       const long long fi = f_index(L, d, k, s);
@@ -523,6 +523,60 @@ __device__ __forceinline__ void kick_site(const KickArgs& a, const LatDev& L, in
       } else {
         reinterpret_cast<double2*>(a.out)[fi] = make_double2((double)F.re, (double)F.im);
       }
+    }
+  }
+}
+
+// Scalar force of a general irrep of many components (KICK_SITE_SPLIT_D): a block takes
+// one 32-site block, a lane per site, and its warps split the d components (psi_f, psi_b
+// and w come from memory, so a thread that walks all d alone waits for 9 d loads in turn
+// with few threads beside it).  Measured, whole kicks at SU(3) 12^4, one thread per site
+// and split: 27-plet FP64 154.8 and 148.1 us, FP32 89.3 and 80.0; octet (d = 8) FP64 35.8
+// and 36.5, sextet (d = 6) 31.8 and 32.8: the sum of |phi|^2 over the warps costs more than
+// two components per thread give back, so d <= 8 keeps one thread per site.
+template <int D, typename R>
+__device__ __forceinline__ void kick_site_gen(const KickArgs& a, const LatDev& L, const Work& w) {
+  typedef typename Cmp<R>::t C;
+  constexpr int NW = KICK_BLOCK / 32;
+  __shared__ C part[NW][32];
+  const int lane = threadIdx.x & 31, q = threadIdx.x >> 5, d = a.d;
+  const int s = w.s0 + (lane < w.n ? lane : 0);
+  int x[D], yb[D];
+  coords<D>(L, s, x);
+  const bool live = lane < w.n && in_box<D>(L, x);
+  const R* phi = (const R*)a.phi;
+  const R* psif = (const R*)a.psif;
+  const R* psib = (const R*)a.psib;
+  C n2 = C(0);
+  for (int k = q; k < d; k += NW) n2 += norm2(ldc<C>(phi, f_index(L, d, k, s)));
+  part[q][lane] = n2;
+  __syncthreads();
+  if (!live) return;
+  n2 = C(0);
+#pragma unroll
+  for (int i = 0; i < NW; ++i) n2 += part[i][lane];
+  const C kap2 = C(2) * (C)L.kappa;
+  const C cc = C(1) + C(2) * (C)L.lambda * (n2 - C(1));
+#pragma unroll
+  for (int mu = 0; mu < D; ++mu) yb[mu] = nbwd(L, s, x[mu], mu);
+  for (int k = q; k < d; k += NW) {
+    const long long fi = f_index(L, d, k, s);
+    const cx<C> pk = ldc<C>(phi, fi);
+    cx<C> F;
+    if (a.pot == POT_MULTI) {
+      const double2 wk = a.wpot[fi];
+      F = sub(scale(pk, C(2) * (C)a.mu2), scale(mk<C>((C)wk.x, (C)wk.y), C(2)));
+    } else {
+      F = scale(pk, C(-2) * cc);
+    }
+#pragma unroll
+    for (int mu = 0; mu < D; ++mu)
+      F = add(F, scale(add(ldc<C>(psif, g_index(L, d, mu, k, s)), ldc<C>(psib, g_index(L, d, mu, k, yb[mu]))), kap2));
+    if (a.mode == M_UPDATE) {
+      R* pi = (R*)a.pi;
+      stc<C>(pi, fi, add(ldc_rw<C>(pi, fi), scale(F, (C)a.eps)));
+    } else {
+      reinterpret_cast<double2*>(a.out)[fi] = make_double2((double)F.re, (double)F.im);
     }
   }
 }
@@ -565,13 +619,20 @@ template <int REP> struct KickMinBlocks<double, REP> {
   static constexpr int v = b * 128 / KICK_BLOCK > 0 ? b * 128 / KICK_BLOCK : 1;
 };
 
-// LIN: the table holds linear items (and perhaps tiles); without, tiles only.  An instance
-// of its own: the FP32 kernel at 72 registers lost 1.7% at 16^4 with both forms inside.
-template <int D, int N, typename R, int REP, bool LIN>
+// LIN: the table holds linear items (and perhaps tiles); without, tiles only.  SPLIT: its
+// site items are kick_site_gen's.  Instances of their own: the FP32 kernel at 72 registers
+// lost 1.7% at 16^4 with both link forms inside, the FP64 sextet 2% with both site forms.
+template <int D, int N, typename R, int REP, bool LIN, bool SPLIT>
 __global__ void __launch_bounds__(KICK_BLOCK, KickMinBlocks<R, REP>::v) k_kick(const KickArgs a) {
   pdl_enter();
   const Work w = a.work[blockIdx.x];
   const LatDev& L = a.lats[w.lat];
+  if constexpr (SPLIT) {
+    if (w.mu < 0) {
+      kick_site_gen<D, R>(a, L, w);
+      return;
+    }
+  }
   int s, x[D], mu = w.mu;
   if (LIN && mu >= KICK_LINEAR - 1) {
     // consecutive sites: extents that power-of-two tiles do not divide (rule and figures
@@ -585,7 +646,7 @@ __global__ void __launch_bounds__(KICK_BLOCK, KickMinBlocks<R, REP>::v) k_kick(c
     return;
   }
   if (mu >= 0) kick_link_dispatch<D, N, R, REP>(a, L, mu, s, x);
-  else if (REP != REP_NONE) kick_site<D, N, R, REP>(a, L, s, x);
+  else if (REP != REP_NONE && !SPLIT) kick_site<D, N, R, REP>(a, L, s, x);
 }
 
 // ---------------------------------------------------------------------------
