@@ -77,6 +77,8 @@ constexpr int XS = RG + 1, WS = KC + 4;   // shared-memory strides: transposed s
 constexpr size_t STEP_SMEM = sizeof(float) * ((size_t)KC * XS + TW * WS + 4);
 enum { FORWARD = 0, GRADIENT = 1, TRAIN = 2 };
 
+__device__ __forceinline__ float as_float(float v) { return v; }
+__device__ __forceinline__ float as_float(__nv_bfloat16 v) { return __bfloat162float(v); }
 struct StepArgs {
   int nl, M, mode, nsteps, rows;       // rows: samples per cluster in FORWARD (grid.y splits them)
   int width[MAXL + 1];
@@ -176,9 +178,12 @@ __device__ __forceinline__ void tile_product(float* sx, float* sw, int nrow, int
   }
 }
 
-__device__ __forceinline__ void cluster_barrier() {   // all threads; orders global memory among the cluster's blocks
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+// all threads; orders global and shared memory among the cluster's blocks
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_barrier() {
+  cluster_arrive();
+  cluster_wait();
 }
 
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(TW * 32) k_steps(const StepArgs t) {
@@ -318,6 +323,362 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(TW * 32) k_steps(co
   }
 }
 
+// ---------------------------------------------------------------------------
+// The same steps with everything a network needs in its cluster's shared memory: each block
+// holds its neurons' weight rows, their moments, the columns of the next layer's weights
+// that its neurons feed (for the gradient), and the whole batch's activations and
+// gradients, which the blocks write into one another's memory (st.shared::cluster).  What
+// is left of a step is its cluster barriers and the chains of multiply-adds between them;
+// k_steps goes through L2 for every operand and its stores must drain before each barrier
+// (2.4 us a layer whatever its size).  Five networks 4-128-128-128-3, batch 32, per step:
+// 26 us against 43.  Taken whenever the layout fits 227 KB (hidden width 128: batch
+// up to 64).  Bound: instruction issue of the short chains (40% of issue slots) and the waits
+// at the barriers between them.  The sums run in the same order as there.
+// ---------------------------------------------------------------------------
+constexpr int RT = 512;      // threads
+struct ResLayout {           // offsets in floats
+  int Bp, RS, RH;            // batch rounded up to 32; row strides: floats RS (odd), halves RH (odd words)
+  int dup;                   // the output layer is computed by every block
+  int per[MAXL];             // neurons per block
+  int A0[2], Y[2], ids[2], O;
+  int A[MAXL], G[MAXL], Z[MAXL], Wf[MAXL], bf[MAXL], Wb[MAXL], m1[MAXL], m2[MAXL];
+  int wfs[MAXL], wbs[MAXL];  // row strides of Wf and Wb
+  int total;
+};
+struct ResArgs { StepArgs s; ResLayout L; };
+
+__device__ __forceinline__ unsigned smem_addr(const void* q) { return (unsigned)__cvta_generic_to_shared(q); }
+__device__ __forceinline__ unsigned peer_addr(unsigned local, int rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+// This block's n16 16-byte words at `local` into the same place of every other block of the
+// cluster (written by all threads after a __syncthreads).
+__device__ __forceinline__ void push(const float* local, int n16, int rank) {
+  const unsigned a = smem_addr(local);
+  for (int e = threadIdx.x; e < n16 * (CL - 1); e += blockDim.x) {
+    const int r = e / n16, v = e - r * n16;
+    const float4 q = *reinterpret_cast<const float4*>(local + 4 * v);
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(peer_addr(a, (rank + 1 + r) % CL) + 16 * v), "f"(q.x),
+                 "f"(q.y), "f"(q.z), "f"(q.w)
+                 : "memory");
+  }
+}
+__device__ __forceinline__ float4 ld_peer4(unsigned a) {
+  float4 q;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w) : "r"(a) : "memory");
+  return q;
+}
+__device__ __forceinline__ void copy4(float* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+
+// Columns in pairs (shared memory delivers one operand row per cycle, so a pair's
+// multiply-adds share each load of x) and rows in groups of 32, one unit per warp:
+// init(c) + sum_k W[c][k] x[k][row], k ascending; epi(c, row, sum).
+template <typename T, typename FI, typename FE>
+__device__ __forceinline__ void columns(const T* x, int xs, const float* W, int ws, int nk, int nc, int B, FI init, FE epi) {
+  const int lane = threadIdx.x & 31, rows = (B + 31) / 32, units = (nc + 1) / 2 * rows;
+  for (int u = threadIdx.x >> 5; u < units; u += RT / 32) {
+    const int c = u / rows * 2, row = (u - u / rows * rows) * 32 + lane, c2 = min(c + 1, nc - 1);
+    const T* px = x + row;
+    const float* w0 = W + c * ws;
+    const float* w1 = W + c2 * ws;
+    float a0 = init(c), a1 = init(c2);
+    int k = 0;
+    for (; k + 16 <= nk; k += 16) {
+      float xv[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) xv[q] = as_float(px[(k + q) * xs]);
+#pragma unroll
+      for (int q = 0; q < 16; q += 4) {
+        const float4 v0 = *reinterpret_cast<const float4*>(w0 + k + q), v1 = *reinterpret_cast<const float4*>(w1 + k + q);
+        a0 = fmaf(v0.x, xv[q], a0); a1 = fmaf(v1.x, xv[q], a1);
+        a0 = fmaf(v0.y, xv[q + 1], a0); a1 = fmaf(v1.y, xv[q + 1], a1);
+        a0 = fmaf(v0.z, xv[q + 2], a0); a1 = fmaf(v1.z, xv[q + 2], a1);
+        a0 = fmaf(v0.w, xv[q + 3], a0); a1 = fmaf(v1.w, xv[q + 3], a1);
+      }
+    }
+    for (; k < nk; ++k) {
+      const float xk = as_float(px[k * xs]);
+      a0 = fmaf(w0[k], xk, a0);
+      a1 = fmaf(w1[k], xk, a1);
+    }
+    if (row < B) {
+      epi(c, row, a0);
+      if (c2 > c) epi(c2, row, a1);
+    }
+  }
+}
+// Weight gradients of neurons in pairs, lanes along the inputs in groups of 64: sum_b G[c][b]
+// x[i][b], b ascending; epi(c, i, sum) and, once per neuron, bias(c, sum_b G[c][b]).
+template <typename T, typename FE, typename FB>
+__device__ __forceinline__ void weight_sums(const T* x, int xs, const float* G, int gs, int B, int nin, int nc, FE epi, FB bias) {
+  const int lane = threadIdx.x & 31, blocks = (nin + 63) / 64, units = (nc + 1) / 2 * blocks;
+  for (int u = threadIdx.x >> 5; u < units; u += RT / 32) {
+    const int c = u / blocks * 2, ib = (u - u / blocks * blocks) * 64, c2 = min(c + 1, nc - 1);
+    const int i0 = min(ib + lane, nin - 1), i1 = min(ib + lane + 32, nin - 1);
+    const T* x0 = x + i0 * xs;
+    const T* x1 = x + i1 * xs;
+    const float* g0 = G + c * gs;
+    const float* g1 = G + c2 * gs;
+    float a00 = 0.f, a01 = 0.f, a10 = 0.f, a11 = 0.f, b0 = 0.f, b1 = 0.f;
+    int b = 0;
+    for (; b + 8 <= B; b += 8) {
+      float p[8], q[8], e[8], f[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) { p[k] = as_float(x0[b + k]); q[k] = as_float(x1[b + k]); e[k] = g0[b + k]; f[k] = g1[b + k]; }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        a00 = fmaf(e[k], p[k], a00); a01 = fmaf(e[k], q[k], a01); b0 = fmaf(e[k], 1.f, b0);
+        a10 = fmaf(f[k], p[k], a10); a11 = fmaf(f[k], q[k], a11); b1 = fmaf(f[k], 1.f, b1);
+      }
+    }
+    for (; b < B; ++b) {
+      const float p = as_float(x0[b]), q = as_float(x1[b]), e = g0[b], f = g1[b];
+      a00 = fmaf(e, p, a00); a01 = fmaf(e, q, a01); b0 = fmaf(e, 1.f, b0);
+      a10 = fmaf(f, p, a10); a11 = fmaf(f, q, a11); b1 = fmaf(f, 1.f, b1);
+    }
+    const bool in0 = ib + lane < nin, in1 = ib + lane + 32 < nin;
+    if (in0) epi(c, i0, a00);
+    if (in1) epi(c, i1, a01);
+    if (c2 > c && in0) epi(c2, i0, a10);
+    if (c2 > c && in1) epi(c2, i1, a11);
+    if (ib == 0 && lane == 0) {
+      bias(c, b0);
+      if (c2 > c) bias(c2, b1);
+    }
+  }
+}
+
+// BP: the batch rounded up to 32, 32 or 64 (row strides are then immediate offsets), or 0: any.
+template <int BP>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(RT, 1) k_steps_resident(const __grid_constant__ ResArgs ar) {
+  extern __shared__ float smem[];
+  const StepArgs& t = ar.s;
+  const ResLayout& L = ar.L;
+  const int rank = blockIdx.x % CL, m = blockIdx.x / CL, nl = t.nl, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NW = RT / 32;
+  const int RS = BP ? BP + 1 : L.RS, RH = BP ? BP + 2 : L.RH;
+  const auto nc4 = [](int n) { return (n + 3) / 4 * 4; };
+  const int n0 = t.width[0], no = t.width[nl];
+  const auto owned = [&](int l, int& c0) {      // this block's neurons of layer l: the first and how many
+    if (L.dup && l == nl - 1) { c0 = 0; return t.width[l + 1]; }
+    c0 = min(t.width[l + 1], rank * L.per[l]);
+    return min(L.per[l], t.width[l + 1] - c0);
+  };
+  // the weights and moments
+  for (int l = 0; l < nl; ++l) {
+    int c0;
+    const int nc = owned(l, c0), nin = t.width[l];
+    const long w = m * t.P + t.woff[l] + (long)c0 * nin, b = m * t.P + t.boff[l] + c0;
+    for (int c = warp; c < nc; c += NW)
+      for (int i = lane; i < nin; i += 32) {
+        smem[L.Wf[l] + c * L.wfs[l] + i] = t.p[w + (long)c * nin + i];
+        smem[L.m1[l] + c * (nin + 1) + i] = t.m1[w + (long)c * nin + i];
+        smem[L.m2[l] + c * (nin + 1) + i] = t.m2[w + (long)c * nin + i];
+      }
+    for (int c = tid; c < nc; c += RT) {
+      smem[L.bf[l] + c] = t.p[b + c];
+      smem[L.m1[l] + c * (nin + 1) + nin] = t.m1[b + c];
+      smem[L.m2[l] + c * (nin + 1) + nin] = t.m2[b + c];
+    }
+  }
+  // columns of layer l's weights that this block's neurons of layer l - 1 feed, from the
+  // blocks that hold the rows
+  const auto pull = [&]() {
+    for (int l = 1; l < nl; ++l) {
+      int i0;
+      const int ni = owned(l - 1, i0), q4 = (ni + 3) / 4, nout = t.width[l + 1];
+      if (q4 == 0) continue;
+      for (int e = tid; e < nout * q4; e += RT) {
+        const int k = e / q4, i = 4 * (e - k * q4), own = L.dup && l == nl - 1 ? rank : k / L.per[l];
+        const int row = L.dup && l == nl - 1 ? k : k - own * L.per[l];
+        const float4 v = ld_peer4(peer_addr(smem_addr(smem + L.Wf[l] + row * L.wfs[l] + i0 + i), own));
+        float* d = smem + L.Wb[l] + i * L.wbs[l] + k;
+        d[0] = v.x;
+        if (i + 1 < ni) d[L.wbs[l]] = v.y;
+        if (i + 2 < ni) d[2 * L.wbs[l]] = v.z;
+        if (i + 3 < ni) d[3 * L.wbs[l]] = v.w;
+      }
+    }
+  };
+  // a step's samples, in flight while the step before it runs
+  const auto info = [&](int st) { return st < t.nsteps ? t.steps[st] : StepInfo{0, 0, -1, 0.f, 0.f}; };
+  const auto fetch_ids = [&](int st, const StepInfo& q) {
+    int* d = reinterpret_cast<int*>(smem + L.ids[st & 1]);
+    for (int b = tid; b < q.B; b += RT) {
+      if (t.idx) copy4(reinterpret_cast<float*>(d + b), t.idx + q.s0 + b);
+      else d[b] = q.s0 + b;
+    }
+  };
+  const auto fetch_samples = [&](int st, int B) {
+    const int* id = reinterpret_cast<const int*>(smem + L.ids[st & 1]);
+    for (int b = warp; b < B; b += NW) {
+      const long q = id[b];
+      for (int k = lane; k < n0; k += 32) copy4(smem + L.A0[st & 1] + k * RS + b, t.x + q * n0 + k);
+      for (int k = lane; k < no; k += 32) copy4(smem + L.Y[st & 1] + k * RS + b, t.y + q * no + k);
+    }
+  };
+  const auto landed = [&]() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+  };
+  StepInfo si = info(0), s1 = info(1), s2 = info(2);   // read ahead of their use
+  fetch_ids(0, si);
+  landed();
+  fetch_samples(0, si.B);
+  fetch_ids(1, s1);
+  landed();
+  cluster_barrier();                            // every block of the cluster runs: its memory may be written
+  for (int st = 0; st < t.nsteps; ++st) {
+    const StepInfo s3 = info(st + 3);
+    const int B = si.B;
+    const float* A0 = smem + L.A0[st & 1];
+    const float* Y = smem + L.Y[st & 1];
+    fetch_samples(st + 1, s1.B);
+    fetch_ids(st + 2, s2);
+    pull();                                     // before the first barrier of the step: Adam comes after it
+    for (int l = 0; l < nl; ++l) {
+      int c0;
+      const int nc = owned(l, c0), nin = t.width[l];
+      const bool last = l == nl - 1;
+      const auto I = [&](int c) { return smem[L.bf[l] + c]; };
+      const auto E = [&](int c, int b, float v) {
+        const int o = (c0 + c) * RS + b;
+        if (!last) {
+          smem[L.Z[l] + c * RS + b] = v;
+          reinterpret_cast<__nv_bfloat16*>(smem + L.A[l + 1])[(c0 + c) * RH + b] = __float2bfloat16(silu(v));
+        } else {
+          const float d = v - Y[o];
+          smem[L.G[l] + o] = 2.f * d / (float)(B * no);
+          smem[L.O + o] = v;
+        }
+      };
+      if (l) columns(reinterpret_cast<const __nv_bfloat16*>(smem + L.A[l]), RH, smem + L.Wf[l], L.wfs[l], nin, nc, B, I, E);
+      else columns(A0, RS, smem + L.Wf[l], L.wfs[l], nin, nc, B, I, E);
+      __syncthreads();
+      if (last && L.dup) break;
+      if (!last) {
+        push(smem + L.A[l + 1] + c0 * RH / 2, nc4(nc) * RH / 8, rank);
+      } else {
+        push(smem + L.G[l] + c0 * RS, nc4(nc) * RS / 4, rank);
+        push(smem + L.O + c0 * RS, nc4(nc) * RS / 4, rank);
+      }
+      cluster_barrier();
+    }
+    for (int l = nl - 1; l > 0; --l) {          // gradient through layer l and the SiLU before it
+      int i0;
+      const int ni = owned(l - 1, i0);
+      columns(smem + L.G[l], RS, smem + L.Wb[l], L.wbs[l], t.width[l + 1], ni, B, [](int) { return 0.f; },
+              [&](int i, int b, float v) {
+        smem[L.G[l - 1] + ((l == 1 ? 0 : i0) + i) * RS + b] = v * dsilu(smem[L.Z[l - 1] + i * RS + b]);
+      });
+      __syncthreads();
+      if (l == 1) break;                        // only this block's weight gradients read G[0]
+      push(smem + L.G[l - 1] + i0 * RS, nc4(ni) * RS / 4, rank);
+      cluster_barrier();
+    }
+    if (si.slot >= 0 && rank == 0 && warp < 8) {  // loss: mean of (out - y)^2, 256 strided sums and a tree
+      float* sh = smem + L.O + (no + 3) / 4 * 4 * RS;
+      float sum = 0.f;
+      for (int e = tid; e < B * no; e += 256) {
+        const float d = smem[L.O + (e % no) * RS + e / no] - Y[(e % no) * RS + e / no];
+        sum += d * d;
+      }
+      sh[tid] = sum;
+      for (int q = 128; q > 0; q >>= 1) {
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (tid < q) sh[tid] += sh[tid + q];
+      }
+      if (tid == 0) t.loss[(long)si.slot * t.M + m] = sh[0] / (float)(B * no);
+    }
+    const bool keep = st == t.nsteps - 1;       // the gradients of the last step stay for gh_mlp_adam_step
+    for (int l = 0; l < nl; ++l) {
+      int c0;
+      const int nc = owned(l, c0), nin = t.width[l];
+      const bool out = keep && (rank == 0 || !(L.dup && l == nl - 1));
+      const auto E = [&](int c, int i, float v) {
+        if (out) t.g[m * t.P + t.woff[l] + (long)(c0 + c) * nin + i] = v;
+        if (t.mode == TRAIN)
+          adam_update(smem + L.Wf[l] + c * L.wfs[l] + i, smem + L.m1[l] + c * (nin + 1) + i, smem + L.m2[l] + c * (nin + 1) + i, v,
+                      t.lr, t.b1, t.b2, t.eps, si.c1, si.c2);
+      };
+      const auto EB = [&](int c, float v) {
+        if (out) t.g[m * t.P + t.boff[l] + c0 + c] = v;
+        if (t.mode == TRAIN)
+          adam_update(smem + L.bf[l] + c, smem + L.m1[l] + c * (nin + 1) + nin, smem + L.m2[l] + c * (nin + 1) + nin, v, t.lr, t.b1,
+                      t.b2, t.eps, si.c1, si.c2);
+      };
+      // G[0] below other layers holds this block's rows only
+      const float* g = smem + L.G[l] + (l || nl == 1 ? c0 : 0) * RS;
+      if (l) weight_sums(reinterpret_cast<const __nv_bfloat16*>(smem + L.A[l]), RH, g, RS, B, nin, nc, E, EB);
+      else weight_sums(A0, RS, g, RS, B, nin, nc, E, EB);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    cluster_barrier();                          // new weights and the next step's samples are in place
+    si = s1;
+    s1 = s2;
+    s2 = s3;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  if (t.mode == TRAIN)
+    for (int l = 0; l < nl; ++l) {
+      int c0;
+      const int nc = owned(l, c0), nin = t.width[l];
+      if (L.dup && l == nl - 1 && rank != 0) break;
+      const long w = m * t.P + t.woff[l] + (long)c0 * nin, b = m * t.P + t.boff[l] + c0;
+      for (int c = warp; c < nc; c += NW)
+        for (int i = lane; i < nin; i += 32) {
+          t.p[w + (long)c * nin + i] = smem[L.Wf[l] + c * L.wfs[l] + i];
+          t.m1[w + (long)c * nin + i] = smem[L.m1[l] + c * (nin + 1) + i];
+          t.m2[w + (long)c * nin + i] = smem[L.m2[l] + c * (nin + 1) + i];
+        }
+      for (int c = tid; c < nc; c += RT) {
+        t.p[b + c] = smem[L.bf[l] + c];
+        t.m1[b + c] = smem[L.m1[l] + c * (nin + 1) + nin];
+        t.m2[b + c] = smem[L.m2[l] + c * (nin + 1) + nin];
+      }
+    }
+}
+
+// The layout for batches of up to maxB samples; false if it does not fit a block.
+bool res_layout(const Net& n, int maxB, ResLayout& L) {
+  std::memset(&L, 0, sizeof(L));
+  long at = 0;
+  const auto take = [&](long f) {               // rows that are read as float4 start on 16 bytes
+    const long o = at;
+    at += (f + 3) / 4 * 4;
+    return (int)std::min<long>(o, 1 << 28);
+  };
+  const auto up4 = [](int x) { return (x + 3) / 4 * 4; };
+  L.Bp = (maxB + 31) / 32 * 32;
+  L.RS = L.Bp + 1;
+  L.RH = L.Bp + 2;
+  const int nl = n.nl, no = n.width[nl];
+  L.dup = no <= 16;
+  for (int k = 0; k < 2; ++k) { L.A0[k] = take((long)n.width[0] * L.RS); L.Y[k] = take((long)no * L.RS); L.ids[k] = take(L.Bp); }
+  L.O = take((long)up4(no) * L.RS + 256);
+  for (int l = 0; l < nl; ++l) {
+    const int nin = n.width[l], nout = n.width[l + 1];
+    const bool dup = L.dup && l == nl - 1;
+    L.per[l] = dup ? nout : up4((nout + CL - 1) / CL);   // fours: slices of A, G and W rows start on 16 bytes
+    const long nc = L.per[l];
+    if (l) L.A[l] = take((long)up4(nin) * L.RH / 2);
+    L.G[l] = take((long)(l || nl == 1 ? up4(nout) : nc) * L.RS);
+    if (l + 1 < nl) L.Z[l] = take(nc * L.RS);
+    L.wfs[l] = up4(nin) + 4;
+    L.Wf[l] = take(nc * L.wfs[l]);
+    L.bf[l] = take(nc);
+    if (l) { L.wbs[l] = up4(nout) + 4; L.Wb[l] = take((long)L.per[l - 1] * L.wbs[l]); }
+    L.m1[l] = take(nc * (nin + 1));
+    L.m2[l] = take(nc * (nin + 1));
+  }
+  L.total = (int)std::min<long>(at, 1 << 28);
+  return at * sizeof(float) <= 227 * 1024;
+}
+
 __global__ void k_adam(float* p, const float* g, float* m1, float* m2, long n, float lr, float b1, float b2, float eps,
                        float c1, float c2) {
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x)
@@ -400,6 +761,18 @@ int run_steps(Net* n, int mode, const std::vector<StepInfo>& steps, const std::v
   t.x = n->xd; t.y = n->yd; t.idx = order ? n->idx : nullptr;
   t.out = n->out; t.loss = n->loss; t.steps = n->steps;
   t.lr = lr; t.b1 = 0.9f; t.b2 = 0.999f; t.eps = 1e-8f;
+  int maxB = 0;
+  for (const StepInfo& q : steps) maxB = std::max(maxB, q.B);
+  ResArgs ra;
+  if (mode != FORWARD && res_layout(*n, maxB, ra.L)) {
+    void (*const k)(ResArgs) = ra.L.Bp == 32 ? k_steps_resident<32> : ra.L.Bp == 64 ? k_steps_resident<64> : k_steps_resident<0>;
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, ra.L.total * (int)sizeof(float));
+    ra.s = t;
+    if (!e) k<<<n->M * CL, RT, ra.L.total * sizeof(float)>>>(ra);
+    e = e ? e : cudaGetLastError();
+    if (e) return mfail(n, GH_ERR_CUDA, std::string("MLP kernel: ") + cudaGetErrorString(e));
+    return GH_OK;
+  }
   t.rows = 64;                                  // forward rows are independent: clusters of 64 samples
   const int gy = mode == FORWARD ? (steps[0].B + t.rows - 1) / t.rows : 1;
   k_steps<<<dim3(n->M * CL, gy), TW * 32, STEP_SMEM>>>(t);
