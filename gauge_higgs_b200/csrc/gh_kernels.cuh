@@ -199,6 +199,23 @@ __device__ __forceinline__ Mat<N, C> ld_link(const R* __restrict__ U, const LatD
   for (int c = 0; c < N * N; ++c) M.e[c] = ldc<C>(U, base + c * ULANE);
   return M;
 }
+// An SU(N) link for the force: SU(2) from its first row (a, b), the second is (-conj b,
+// conj a) -- half the loads, and the products below use one row (kick of a ladder of 16
+// SU(2) lattices of 6, 8, 10, 12: FP32 34.3 -> 18.8 us, FP64 60.3 -> 28.6 us).  Other
+// N: every entry.
+template <int N, typename C, typename R>
+__device__ __forceinline__ Mat<N, C> ld_su(const R* __restrict__ U, const LatDev& L, int mu, int s) {
+  if constexpr (N == 2) {
+    Mat<N, C> M;
+    const long long base = u_index(L, N * N, mu, 0, s);
+    M.e[0] = ldc<C>(U, base);
+    M.e[1] = ldc<C>(U, base + ULANE);
+    su2_second_row(M);
+    return M;
+  } else {
+    return ld_link<N, C>(U, L, mu, s);
+  }
+}
 template <int N, typename C, typename R>
 __device__ __forceinline__ Mat<N, C> ld_link_rw(const R* U, const LatDev& L, int mu, int s) {
   Mat<N, C> M;
@@ -333,7 +350,10 @@ __device__ __forceinline__ void kick_link(const KickArgs& a, const LatDev& L, in
   Mat<N, C> Om;
   set_zero(Om);
   Mat<N, C> Umu;
-  if (!(a.flags & F_GAUGE)) Umu = ld_link<N, C>(U, L, mu, s);
+  // rows of the staple sum: a real combination of SU(2) matrices has the form of one, so its
+  // first row is all of it
+  constexpr int ROWS = N == 2 ? 1 : N;
+  if (!(a.flags & F_GAUGE)) Umu = ld_su<N, C>(U, L, mu, s);
   if (a.flags & F_GAUGE) {
     Mat<N, C> sig;
     set_zero(sig);
@@ -345,16 +365,18 @@ __device__ __forceinline__ void kick_link(const KickArgs& a, const LatDev& L, in
       const int spm_mn = nbwd(L, spm, x[nu], nu);
       // upper staple U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag, lower U_nu(x+mu-nu)^dag U_mu(x-nu)^dag U_nu(x-nu)
       // (the inner products of two links through mm_su: their last row from unitarity)
-      mm_nd_acc(sig, mm_su<N, C, false, true>(ld_link<N, C>(U, L, nu, spm), ld_link<N, C>(U, L, mu, spn)),
-                ld_link<N, C>(U, L, nu, s));
-      mm_acc(sig, mm_su<N, C, true, true>(ld_link<N, C>(U, L, nu, spm_mn), ld_link<N, C>(U, L, mu, smn)),
-             ld_link<N, C>(U, L, nu, smn));
+      mm_core<N, C, false, true, true, ROWS>(mm_su<N, C, false, true>(ld_su<N, C>(U, L, nu, spm), ld_su<N, C>(U, L, mu, spn)),
+                                             ld_su<N, C>(U, L, nu, s), sig);
+      mm_core<N, C, false, false, true, ROWS>(mm_su<N, C, true, true>(ld_su<N, C>(U, L, nu, spm_mn), ld_su<N, C>(U, L, mu, smn)),
+                                              ld_su<N, C>(U, L, nu, smn), sig);
     }
-    Umu = ld_link<N, C>(U, L, mu, s);
-    Om = mm(Umu, sig);
+    if constexpr (N == 2) su2_second_row(sig);
+    Umu = ld_su<N, C>(U, L, mu, s);
+    mm_core<N, C, false, false, false, ROWS>(Umu, sig, Om);
     const C c = (C)(L.beta / N);
 #pragma unroll
-    for (int i = 0; i < N * N; ++i) Om.e[i] = scale(Om.e[i], c);
+    for (int i = 0; i < ROWS * N; ++i) Om.e[i] = scale(Om.e[i], c);
+    if constexpr (N == 2) su2_second_row(Om);
   }
   if ((a.flags & F_MATTER) && (REP == REP_FUND || REP == REP_ADJ)) {
     constexpr int d = RepDim<N, REP>::d;
@@ -470,13 +492,13 @@ __device__ __forceinline__ void kick_site(const KickArgs& a, const LatDev& L, in
 #pragma unroll
       for (int k = 0; k < d; ++k) v[k] = ldc<C>(phi, f_index(L, d, k, yf));
       {
-        const Mat<N, C> Uf = ld_link<N, C>(U, L, mu, s);
+        const Mat<N, C> Uf = ld_su<N, C>(U, L, mu, s);
         if (REP == REP_FUND) fund_apply<N, C>(Uf, v, o, false); else adj_apply<N, C>(Uf, v, o, false);
       }
 #pragma unroll
       for (int k = 0; k < d; ++k) v[k] = ldc<C>(phi, f_index(L, d, k, yb));
       {
-        const Mat<N, C> Ub = ld_link<N, C>(U, L, mu, yb);
+        const Mat<N, C> Ub = ld_su<N, C>(U, L, mu, yb);
         if (REP == REP_FUND) fund_apply<N, C>(Ub, v, o2, true); else adj_apply<N, C>(Ub, v, o2, true);
       }
 #pragma unroll
@@ -599,11 +621,20 @@ __device__ __forceinline__ void kick_link_dispatch(const KickArgs& a, const LatD
 // us) and at FP64 3 and 4 (40.7 / 40.9 us), while the trajectory with the higher
 // occupancy is 1.4% (FP32) and 1.7% (FP64) faster -- the next launch's blocks find room
 // sooner; FP32 6 blocks (80 registers) was 2.5% slower; FP32 4 / FP64 2 lose ~4%.
+// SU(2) (links from their first row, ld_su): FP32 8 and FP64 5.  A ladder of 16 lattices of
+// 6, 8, 10, 12 / one 6^4, trajectories in us: FP32 7 blocks 1184 / 126, 8 1134 / 124, 9 1128 /
+// 126; FP64 4 1851 / 141, 5 1702 / 138, 6 (spills) 1674 / 144.
 #ifndef GH_KICK_MINB_F32
 #define GH_KICK_MINB_F32 5
 #endif
 #ifndef GH_KICK_MINB_F32_FUND
 #define GH_KICK_MINB_F32_FUND 7
+#endif
+#ifndef GH_KICK_MINB_F32_SU2
+#define GH_KICK_MINB_F32_SU2 8
+#endif
+#ifndef GH_KICK_MINB_F64_SU2
+#define GH_KICK_MINB_F64_SU2 5
 #endif
 #ifndef GH_KICK_MINB_F64
 #define GH_KICK_MINB_F64 3
@@ -611,11 +642,12 @@ __device__ __forceinline__ void kick_link_dispatch(const KickArgs& a, const LatD
 #ifndef GH_KICK_MINB_F64_FUND
 #define GH_KICK_MINB_F64_FUND 4
 #endif
-template <typename R, int REP> struct KickMinBlocks {
-  static constexpr int v = (REP == REP_FUND ? GH_KICK_MINB_F32_FUND : GH_KICK_MINB_F32) * 128 / KICK_BLOCK;
+template <int N, typename R, int REP> struct KickMinBlocks {
+  static constexpr int b = N == 2 ? GH_KICK_MINB_F32_SU2 : REP == REP_FUND ? GH_KICK_MINB_F32_FUND : GH_KICK_MINB_F32;
+  static constexpr int v = b * 128 / KICK_BLOCK;
 };
-template <int REP> struct KickMinBlocks<double, REP> {
-  static constexpr int b = REP == REP_FUND ? GH_KICK_MINB_F64_FUND : GH_KICK_MINB_F64;
+template <int N, int REP> struct KickMinBlocks<N, double, REP> {
+  static constexpr int b = N == 2 ? GH_KICK_MINB_F64_SU2 : REP == REP_FUND ? GH_KICK_MINB_F64_FUND : GH_KICK_MINB_F64;
   static constexpr int v = b * 128 / KICK_BLOCK > 0 ? b * 128 / KICK_BLOCK : 1;
 };
 
@@ -623,7 +655,7 @@ template <int REP> struct KickMinBlocks<double, REP> {
 // site items are kick_site_gen's.  Instances of their own: the FP32 kernel at 72 registers
 // lost 1.7% at 16^4 with both link forms inside, the FP64 sextet 2% with both site forms.
 template <int D, int N, typename R, int REP, bool LIN, bool SPLIT>
-__global__ void __launch_bounds__(KICK_BLOCK, KickMinBlocks<R, REP>::v) k_kick(const KickArgs a) {
+__global__ void __launch_bounds__(KICK_BLOCK, KickMinBlocks<N, R, REP>::v) k_kick(const KickArgs a) {
   pdl_enter();
   const Work w = a.work[blockIdx.x];
   const LatDev& L = a.lats[w.lat];

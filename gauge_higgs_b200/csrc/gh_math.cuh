@@ -152,6 +152,11 @@ template <typename T> GH_HD cx<T> conj_cross(const cx<T>& a, const cx<T>& b, con
   im = fmad(-a.im, b.re, im);
   return mk<T>(re, im);
 }
+// The second row of a matrix of SU(2) form (a real multiple of one) from its first.
+template <typename T> GH_HD void su2_second_row(Mat<2, T>& M) {
+  M.e[2] = mk<T>(-M.e[1].re, M.e[1].im);
+  M.e[3] = mk<T>(M.e[0].re, -M.e[0].im);
+}
 // Product of two SU(N) matrices, N = 2 or 3: the first N-1 rows as products, the last
 // from them through unitarity and det = 1 (SU(3): row 2 = conj(row 0 x row 1); SU(2):
 // row 1 = (-conj c01, conj c00)).  The last row costs 24 multiply-adds instead of 36
@@ -168,8 +173,7 @@ template <int N, typename T, bool DA, bool DB> GH_HD Mat<N, T> mm_su(const Mat<N
     C.e[8] = conj_cross(C.e[0], C.e[4], C.e[1], C.e[3]);
   } else if constexpr (N == 2) {
     mm_core<N, T, DA, DB, false, 1>(A, B, C);
-    C.e[2] = mk<T>(-C.e[1].re, C.e[1].im);
-    C.e[3] = mk<T>(C.e[0].re, -C.e[0].im);
+    su2_second_row(C);
   } else {
     mm_core<N, T, DA, DB, false>(A, B, C);
   }
@@ -431,12 +435,34 @@ template <typename T> GH_HD Mat<2, T> expi2(const Mat<2, T>& H) {
 #pragma unroll
     for (int k = 0; k < 2; ++k) trh2 += mul(H.e[i * 2 + k], H.e[k * 2 + i]).re;
   const T r2 = T(0.5) * trh2;
-  const T r = sqrt(r2 > T(0) ? r2 : T(0));
   T c, sinc;
-  // below the cut-off the next terms of cos r and sin(r)/r are under the type's resolution
-  const T rsmall = sizeof(T) == sizeof(double) ? T(1e-8) : T(1e-4);
-  if (r < rsmall) { c = T(1) - T(0.5) * r2; sinc = T(1) - r2 / T(6); }
-  else { T sn; sincos(r, &sn, &c); sinc = sn / r; }
+  if (r2 <= T(0.25)) {
+    // Taylor series in r^2 of cos r and sin(r)/r: for r <= 1/2 (an MD step has r ~ 0.05) the
+    // terms past r^16 / 16! are below 1e-18 -- no square root, division or range reduction
+    c = T(1.0 / 20922789888000.0);
+    c = fmad(c, r2, T(-1.0 / 87178291200.0));
+    c = fmad(c, r2, T(1.0 / 479001600.0));
+    c = fmad(c, r2, T(-1.0 / 3628800.0));
+    c = fmad(c, r2, T(1.0 / 40320.0));
+    c = fmad(c, r2, T(-1.0 / 720.0));
+    c = fmad(c, r2, T(1.0 / 24.0));
+    c = fmad(c, r2, T(-0.5));
+    c = fmad(c, r2, T(1));
+    sinc = T(1.0 / 355687428096000.0);
+    sinc = fmad(sinc, r2, T(-1.0 / 1307674368000.0));
+    sinc = fmad(sinc, r2, T(1.0 / 6227020800.0));
+    sinc = fmad(sinc, r2, T(-1.0 / 39916800.0));
+    sinc = fmad(sinc, r2, T(1.0 / 362880.0));
+    sinc = fmad(sinc, r2, T(-1.0 / 5040.0));
+    sinc = fmad(sinc, r2, T(1.0 / 120.0));
+    sinc = fmad(sinc, r2, T(-1.0 / 6.0));
+    sinc = fmad(sinc, r2, T(1));
+  } else {
+    const T r = sqrt(r2);
+    T sn;
+    sincos(r, &sn, &c);
+    sinc = sn / r;
+  }
   Mat<2, T> U;
 #pragma unroll
   for (int i = 0; i < 4; ++i) U.e[i] = mk<T>(-sinc * H.e[i].im, sinc * H.e[i].re);
