@@ -40,6 +40,10 @@ struct gh_ctx {
   int use_graph = 1;
   double* staging = nullptr;
   size_t staging_elems = 0;
+  // pinned host memory for small results (records, partial sums): a copy into it neither
+  // stages nor blocks, so one synchronise ends a call.  Grows to the largest result.
+  void* pin = nullptr;
+  size_t pin_cap = 0;
   double* fbuf = nullptr;             // FP64 SoA force output (links)
   double* fphibuf = nullptr;          // FP64 SoA force output (vectors)
   std::vector<void*> allocs;
@@ -91,6 +95,7 @@ struct gh_ctx {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (graph) cudaGraphDestroy(graph);
     for (void* p : allocs) cudaFree(p);
+    if (pin) cudaFreeHost(pin);
     if (own) cudaStreamDestroy(own);
   }
 };
@@ -122,6 +127,20 @@ int dalloc(gh_ctx* ctx, T** p, size_t n) {
   ctx->allocs.push_back(q);
   ctx->bytes += bytes;
   *p = (T*)q;
+  return GH_OK;
+}
+
+int pinned(gh_ctx* ctx, size_t bytes, void** p) {
+  if (bytes > ctx->pin_cap) {
+    CK(cudaStreamSynchronize(ctx->st));
+    if (ctx->pin) cudaFreeHost(ctx->pin);
+    ctx->pin = nullptr;
+    ctx->pin_cap = 0;
+    const size_t cap = std::max<size_t>(2 * bytes, 1 << 16);
+    CK(cudaHostAlloc(&ctx->pin, cap, cudaHostAllocDefault));
+    ctx->pin_cap = cap;
+  }
+  *p = ctx->pin;
   return GH_OK;
 }
 
@@ -234,7 +253,7 @@ void enq_trajectory(gh_ctx* ctx) {
   if (ctx->prec == GH_PREC_FP64) ctx->eng->reunit(b);
   enq_measure(ctx, 1);
   MetroArgs m;
-  m.lats = b.lats; m.res = b.res; m.hist = b.hist; m.hist_cap = b.hist_cap; m.nlat = ctx->nlat; m.pure = ctx->scalar ? 0 : 1;
+  m.lats = b.lats; m.res = b.res; m.hist = b.hist; m.hist_cap = b.hist_cap; m.last = b.last; m.nlat = ctx->nlat; m.pure = ctx->scalar ? 0 : 1;
   launch(k_metropolis, (ctx->nlat + 63) / 64, 64, 0, ctx->st, m);
   ctx->eng->restore(b);
   if (ctx->temper && (ctx->scalar || ctx->temper == 2)) {
@@ -270,6 +289,60 @@ int run_traj(gh_ctx* ctx) {
     enq_trajectory(ctx);
   }
   return launch_check(ctx, "trajectory");
+}
+
+gh_traj_record to_record(const TrajRec& r) {
+  gh_traj_record o;
+  o.dH = r.dH; o.accepted = r.accepted; o.traj = r.traj; o.plaquette = r.plaq; o.L_phi = r.L_phi; o.L_link = r.L_link;
+  o.kappa = r.kappa; o.beta = r.beta;
+  return o;
+}
+
+// The records of the trajectory enqueued last, one per lattice: k_metropolis keeps them
+// beside the ring, so no counter has to be read first.
+int fetch_last(gh_ctx* ctx, gh_traj_record* out) {
+  void* pin;
+  int rc = pinned(ctx, sizeof(TrajRec) * ctx->nlat, &pin);
+  if (rc) return rc;
+  CK(cudaMemcpyAsync(pin, ctx->b.last, sizeof(TrajRec) * ctx->nlat, cudaMemcpyDeviceToHost, ctx->st));
+  CK(cudaStreamSynchronize(ctx->st));
+  for (int l = 0; l < ctx->nlat; ++l) out[l] = to_record(((const TrajRec*)pin)[l]);
+  return GH_OK;
+}
+
+// The records of the last n (<= ring size) trajectories into out, [trajectory][lattice];
+// zeros where a lattice's counter says that there was none.  The counters first (on the
+// device: a caller may replay captured trajectories), then the records asked for only.
+int fetch_records(gh_ctx* ctx, int n, gh_traj_record* out) {
+  if (n == 0) return GH_OK;
+  const int cap = ctx->b.hist_cap, nl = ctx->nlat;
+  const size_t nrec = (size_t)nl * n;
+  void* pin;
+  int rc = pinned(ctx, sizeof(TrajRec) * nrec + sizeof(unsigned long long) * nl, &pin);
+  if (rc) return rc;
+  TrajRec* h = (TrajRec*)pin;
+  unsigned long long* traj = (unsigned long long*)(h + nrec);
+  CK(cudaMemcpy2DAsync(traj, sizeof(unsigned long long), (const char*)ctx->b.lats + offsetof(LatDev, traj), sizeof(LatDev),
+                       sizeof(unsigned long long), nl, cudaMemcpyDeviceToHost, ctx->st));
+  CK(cudaStreamSynchronize(ctx->st));
+  // lattices in a row whose rings stand at the same slot go in one strided copy
+  for (int l = 0; l < nl;) {
+    int m = 1;
+    while (l + m < nl && traj[l + m] == traj[l]) ++m;
+    const int have = (int)std::min<unsigned long long>(traj[l], (unsigned long long)n);
+    for (int done = 0, k; done < have; done += k) {
+      const int slot = (int)((traj[l] - have + done) % (unsigned long long)cap);
+      k = std::min(have - done, cap - slot);
+      CK(cudaMemcpy2DAsync(h + (size_t)l * n + (n - have) + done, sizeof(TrajRec) * n, ctx->b.hist + (size_t)l * cap + slot,
+                           sizeof(TrajRec) * cap, sizeof(TrajRec) * k, m, cudaMemcpyDeviceToHost, ctx->st));
+    }
+    l += m;
+  }
+  CK(cudaStreamSynchronize(ctx->st));
+  for (int l = 0; l < nl; ++l)
+    for (int t = 0; t < n; ++t)
+      out[(size_t)t * nl + l] = traj[l] < (unsigned long long)(n - t) ? gh_traj_record{} : to_record(h[(size_t)l * n + t]);
+  return GH_OK;
 }
 
 int check_lat(gh_ctx* ctx, int lat, bool allow_all) {
@@ -865,7 +938,7 @@ int gh_ctx_create(int D, int N, int n_lat, const int* L, const gh_rep_desc* rep,
       (rc = dalloc(ctx, &b.w_gen, std::max<size_t>(wg.size(), 1))) ||
       (rc = dalloc(ctx, &b.w_gprod, std::max<size_t>(wgp.size(), 1))) || (rc = dalloc(ctx, &b.blk_first, blk_first.size())) ||
       (rc = dalloc(ctx, &b.partials, (size_t)ws.size() * NRED)) || (rc = dalloc(ctx, &b.res, (size_t)n_lat * 2 * NRES)) ||
-      (rc = dalloc(ctx, &b.hist, (size_t)n_lat * b.hist_cap)) || (rc = dalloc(ctx, &ctx->staging, stage)) ||
+      (rc = dalloc(ctx, &b.hist, (size_t)n_lat * b.hist_cap)) || (rc = dalloc(ctx, &b.last, n_lat)) || (rc = dalloc(ctx, &ctx->staging, stage)) ||
       (rc = dalloc(ctx, &ctx->fbuf, (size_t)std::max<long long>(p, 1))) ||
       (rc = dalloc(ctx, &ctx->fphibuf, (size_t)std::max<long long>(f, 1) * 2)))
     { g_err = ctx->err; return rc; }
@@ -1117,8 +1190,10 @@ int gh_measure(gh_ctx* ctx, int lat, gh_obs* out) {
   if (!out) return fail(ctx, GH_ERR_ARG, "null output");
   enq_measure(ctx, 0);
   if ((rc = launch_check(ctx, "measure"))) return rc;
-  std::vector<double> res((size_t)ctx->nlat * 2 * NRES);
-  CK(cudaMemcpyAsync(res.data(), ctx->b.res, res.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
+  void* pin;
+  if ((rc = pinned(ctx, sizeof(double) * (size_t)ctx->nlat * 2 * NRES, &pin))) return rc;
+  const double* res = (const double*)pin;
+  CK(cudaMemcpyAsync(pin, ctx->b.res, sizeof(double) * (size_t)ctx->nlat * 2 * NRES, cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
   const int l0 = lat < 0 ? 0 : lat, l1 = lat < 0 ? ctx->nlat : lat + 1;
   for (int l = l0; l < l1; ++l) {
@@ -1132,8 +1207,11 @@ int gh_measure(gh_ctx* ctx, int lat, gh_obs* out) {
 // Per-lattice sums of the per-block partials written by a site-item reduction
 // kernel (site items are laid out per lattice in order), divided by norm[l].
 int site_partials_to_lattices(gh_ctx* ctx, int lat, const std::vector<double>& norm, double* out) {
-  std::vector<double> part(ctx->b.nw_sites);
-  CK(cudaMemcpyAsync(part.data(), ctx->b.partials, part.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
+  void* pin;
+  const int rc = pinned(ctx, ctx->b.nw_sites * sizeof(double), &pin);
+  if (rc) return rc;
+  const double* part = (const double*)pin;
+  CK(cudaMemcpyAsync(pin, ctx->b.partials, ctx->b.nw_sites * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
   int first = 0;
   const int l0 = lat < 0 ? 0 : lat, l1 = lat < 0 ? ctx->nlat : lat + 1;
@@ -1219,23 +1297,9 @@ int gh_polyakov(gh_ctx* ctx, int lat, int tdir, double* out) {
   if (tdir >= ctx->D) return fail(ctx, GH_ERR_ARG, "tdir out of range");
   ctx->eng->polyakov(ctx->b, tdir);
   if ((rc = launch_check(ctx, "polyakov"))) return rc;
-  std::vector<double> part(ctx->b.nw_sites);
-  CK(cudaMemcpyAsync(part.data(), ctx->b.partials, part.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaStreamSynchronize(ctx->st));
-  // blk_first on the host: site items are laid out per lattice in order
-  int first = 0;
-  const int l0 = lat < 0 ? 0 : lat, l1 = lat < 0 ? ctx->nlat : lat + 1;
-  for (int l = 0; l < ctx->nlat; ++l) {
-    const int nb = (ctx->lat_h[l].V + KBLOCK - 1) / KBLOCK;
-    if (l >= l0 && l < l1) {
-      double s = 0.0;
-      for (int q = first; q < first + nb; ++q) s += part[q];
-      const double count = (double)ctx->lat_h[l].V / ctx->lat_h[l].L[tdir];
-      out[l - l0] = s / (count * ctx->N);
-    }
-    first += nb;
-  }
-  return GH_OK;
+  std::vector<double> norm(ctx->nlat);
+  for (int l = 0; l < ctx->nlat; ++l) norm[l] = (double)ctx->lat_h[l].V / ctx->lat_h[l].L[tdir] * ctx->N;
+  return site_partials_to_lattices(ctx, lat, norm, out);
 }
 
 int gh_set_tile(gh_ctx* ctx, int lat, const int* tile) {
@@ -1399,14 +1463,11 @@ int gh_trajectory(gh_ctx* ctx, double* dH, int* accepted) {
   if (!ctx) return fail(nullptr, GH_ERR_ARG, "null context");
   int rc = run_traj(ctx);
   if (rc) return rc;
-  std::vector<LatDev> L(ctx->nlat);
-  std::vector<double> res((size_t)ctx->nlat * 2 * NRES);
-  CK(cudaMemcpyAsync(L.data(), ctx->b.lats, sizeof(LatDev) * ctx->nlat, cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaMemcpyAsync(res.data(), ctx->b.res, res.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaStreamSynchronize(ctx->st));
+  std::vector<gh_traj_record> r(ctx->nlat);
+  if ((rc = fetch_last(ctx, r.data()))) return rc;
   for (int l = 0; l < ctx->nlat; ++l) {
-    if (dH) dH[l] = res[((size_t)l * 2 + 1) * NRES] - res[(size_t)l * 2 * NRES];
-    if (accepted) accepted[l] = L[l].last_acc;
+    if (dH) dH[l] = r[l].dH;
+    if (accepted) accepted[l] = r[l].accepted;
   }
   return GH_OK;
 }
@@ -1415,23 +1476,13 @@ int gh_run_trajectories(gh_ctx* ctx, int ntraj, gh_traj_record* records) {
   if (!ctx) return fail(nullptr, GH_ERR_ARG, "null context");
   if (ntraj < 0) return fail(ctx, GH_ERR_ARG, "ntraj < 0");
   const int cap = ctx->b.hist_cap;
-  std::vector<TrajRec> h((size_t)ctx->nlat * cap);
   for (int t0 = 0; t0 < ntraj; t0 += cap) {
     const int nt = std::min(cap, ntraj - t0);
     for (int t = 0; t < nt; ++t) { int rc = run_traj(ctx); if (rc) return rc; }
     if (records) {
-      std::vector<LatDev> L(ctx->nlat);
-      CK(cudaMemcpyAsync(L.data(), ctx->b.lats, sizeof(LatDev) * ctx->nlat, cudaMemcpyDeviceToHost, ctx->st));
-      CK(cudaMemcpyAsync(h.data(), ctx->b.hist, sizeof(TrajRec) * h.size(), cudaMemcpyDeviceToHost, ctx->st));
-      CK(cudaStreamSynchronize(ctx->st));
-      for (int l = 0; l < ctx->nlat; ++l)
-        for (int t = 0; t < nt; ++t) {
-          const unsigned long long tr = L[l].traj - (unsigned long long)(nt - t);   // traj number - 1 of record t
-          const TrajRec& r = h[(size_t)l * cap + (int)(tr % (unsigned long long)cap)];
-          gh_traj_record& o = records[(size_t)(t0 + t) * ctx->nlat + l];
-          o.dH = r.dH; o.accepted = r.accepted; o.traj = r.traj; o.plaquette = r.plaq; o.L_phi = r.L_phi; o.L_link = r.L_link; o.kappa = r.kappa;
-          o.beta = r.beta;
-        }
+      gh_traj_record* out = records + (size_t)t0 * ctx->nlat;
+      const int rc = nt == 1 ? fetch_last(ctx, out) : fetch_records(ctx, nt, out);
+      if (rc) return rc;
     }
   }
   if (!records) CK(cudaStreamSynchronize(ctx->st));
@@ -1449,21 +1500,7 @@ int gh_read_records(gh_ctx* ctx, int ntraj, gh_traj_record* records) {
   if (!ctx) return fail(nullptr, GH_ERR_ARG, "null context");
   const int cap = ctx->b.hist_cap;
   if (ntraj < 0 || ntraj > cap || !records) return fail(ctx, GH_ERR_ARG, "need 0 <= ntraj <= 1024 and an output array");
-  std::vector<TrajRec> h((size_t)ctx->nlat * cap);
-  std::vector<LatDev> L(ctx->nlat);
-  CK(cudaMemcpyAsync(L.data(), ctx->b.lats, sizeof(LatDev) * ctx->nlat, cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaMemcpyAsync(h.data(), ctx->b.hist, sizeof(TrajRec) * h.size(), cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaStreamSynchronize(ctx->st));
-  for (int l = 0; l < ctx->nlat; ++l)
-    for (int t = 0; t < ntraj; ++t) {
-      gh_traj_record& o = records[(size_t)t * ctx->nlat + l];
-      if (L[l].traj < (unsigned long long)(ntraj - t)) { std::memset(&o, 0, sizeof(o)); continue; }
-      const unsigned long long tr = L[l].traj - (unsigned long long)(ntraj - t);
-      const TrajRec& r = h[(size_t)l * cap + (int)(tr % (unsigned long long)cap)];
-      o.dH = r.dH; o.accepted = r.accepted; o.traj = r.traj; o.plaquette = r.plaq; o.L_phi = r.L_phi; o.L_link = r.L_link; o.kappa = r.kappa;
-          o.beta = r.beta;
-    }
-  return GH_OK;
+  return fetch_records(ctx, ntraj, records);
 }
 
 int gh_trajectory_host(gh_ctx* ctx, double* U, double* phi, gh_traj_record* rec) {
@@ -1475,22 +1512,13 @@ int gh_trajectory_host(gh_ctx* ctx, double* U, double* phi, gh_traj_record* rec)
   if ((rc = run_traj(ctx))) return rc;
   // the record first: a rejected trajectory restores the state that was passed in, so
   // the fields are only copied back when the trajectory was accepted
-  LatDev L;
-  TrajRec r;
-  CK(cudaMemcpyAsync(&L, ctx->b.lats, sizeof(L), cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaStreamSynchronize(ctx->st));
-  const int slot = (int)((L.traj - 1) % (unsigned long long)ctx->b.hist_cap);
-  CK(cudaMemcpyAsync(&r, ctx->b.hist + slot, sizeof(r), cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaStreamSynchronize(ctx->st));
+  gh_traj_record r;
+  if ((rc = fetch_last(ctx, &r))) return rc;
   if (r.accepted) {
     if (U && (rc = gh_get_links(ctx, 0, U))) return rc;
     if (phi && ctx->scalar && (rc = gh_get_phi(ctx, 0, phi))) return rc;
   }
-  if (rec) {
-    rec->dH = r.dH; rec->accepted = r.accepted; rec->traj = r.traj; rec->plaquette = r.plaq; rec->L_phi = r.L_phi; rec->L_link = r.L_link;
-    rec->kappa = r.kappa;
-    rec->beta = r.beta;
-  }
+  if (rec) *rec = r;
   return GH_OK;
 }
 

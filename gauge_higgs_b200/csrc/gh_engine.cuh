@@ -44,6 +44,7 @@ struct Bufs {
   double* partials;
   double* res;
   TrajRec* hist;
+  TrajRec* last;   // [nlat] the last trajectory's record
   int hist_cap;
   GenTables gen;
   Sym2Tab s2tab;

@@ -1850,7 +1850,7 @@ static __global__ void k_finalize(const FinArgs a) {
 // where every comparison with NaN is false) and is counted.  Appends a record.
 // ---------------------------------------------------------------------------
 struct TrajRec { double dH; int accepted; int traj; double plaq, L_phi, L_link, kappa, beta; };
-struct MetroArgs { LatDev* lats; const double* res; TrajRec* hist; int hist_cap; int nlat; int pure; };
+struct MetroArgs { LatDev* lats; const double* res; TrajRec* hist; TrajRec* last; int hist_cap; int nlat; int pure; };
 static __global__ void k_metropolis(const MetroArgs a) {
   pdl_enter();
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1877,6 +1877,7 @@ static __global__ void k_metropolis(const MetroArgs a) {
     h.L_link = ro[6];
     h.kappa = L.kappa;
     h.beta = L.beta;
+    a.last[l] = h;
   }
 }
 
