@@ -605,7 +605,7 @@ int build_general(gh_ctx* ctx, const gh_rep_desc* r) {
   if (!t_j.empty()) CK(cudaMemcpyAsync(p6, t_j.data(), t_j.size() * 4, cudaMemcpyHostToDevice, ctx->st));
   if (!t_v.empty()) CK(cudaMemcpyAsync(v3, t_v.data(), t_v.size() * 16, cudaMemcpyHostToDevice, ctx->st));
   t.wt_ptr = p1; t.wt_l = p2; t.wt_v = v1; t.w_ptr = p3; t.w_i = p4; t.w_v = v2; t.t_ptr = p5; t.t_j = p6; t.t_v = v3;
-  t.sp_ptr = nullptr; t.sp_c = nullptr; t.sp_e = nullptr;
+  t.sp_ptr = nullptr; t.sp_c = nullptr; t.sp_e = nullptr; t.spin_ent = nullptr; t.spin_c = nullptr;
   t.pq64 = nullptr; t.pq32 = nullptr; t.prow = nullptr; t.pnrows = 0; t.pndiag = 0; t.psym = 0; t.s2 = 0;
   // the N x N matrix map: the two-slot basis itself, or the one-fold adjoint product's
   std::vector<std::complex<double>> Wm;
@@ -638,6 +638,50 @@ int build_general(gh_ctx* ctx, const gh_rep_desc* r) {
     CK(cudaMemcpyAsync(sc, q.c.data(), q.c.size() * 8, cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(se, q.off.data(), q.off.size(), cudaMemcpyHostToDevice, ctx->st));   // power-table offsets, word-padded
     t.sp_ptr = sptr; t.sp_c = sc; t.sp_e = se;
+    if (N == 2) {
+      // real sums per entry (k_gen_spin): the term U00^K00 U01^K01 U10^K10 U11^K11 of entry
+      // (k, l), k + l <= n, with U's second row (-conj b, conj a), is (-1)^K10 times
+      // a^(n-k-l) b^(l-k) |a|^2(m-i) |b|^2i, i = K10 (l >= k) or K10 - (k - l)
+      const int n = r->n_boxes;
+      std::vector<int4> ent;
+      std::vector<double> sc2;
+      bool real = d == n + 1;
+      for (int k = 0; k <= n && real; ++k)
+        for (int l = 0; k + l <= n && real; ++l) {
+          const int m = std::min(k, l), e = k * d + l;
+          ent.push_back(make_int4(k, l, (int)sc2.size(), 0));
+          sc2.resize(sc2.size() + m + 1, 0.0);
+          double* sk = &sc2[sc2.size() - m - 1];
+          for (int z = q.ptr[e]; z < q.ptr[e + 1]; ++z) {
+            const int K10 = q.e[(size_t)z * 4 + 2], i = l >= k ? K10 : K10 - (k - l);
+            real = real && i >= 0 && i <= m && q.c[2 * z + 1] == 0.0;
+            if (real) sk[i] += (K10 & 1) ? -q.c[2 * z] : q.c[2 * z];
+          }
+        }
+      // the mirror entries by symmetry: (-1)^(k+l) conj(D_kl) needs the basis to have it
+      const auto mirrored = [&]() {
+        const double th[2] = {0.83, 2.1};
+        for (double t0 : th) {
+          const std::complex<double> u0 = std::polar(std::cos(t0), 0.7 * t0), u1 = std::polar(std::sin(t0), -1.3 * t0);
+          const std::complex<double> U[4] = {u0, u1, -std::conj(u1), std::conj(u0)};
+          std::vector<std::complex<double>> Dm((size_t)d * d);
+          ghsym::eval(q, reinterpret_cast<const double*>(U), reinterpret_cast<double*>(Dm.data()));
+          for (int k = 0; k < d; ++k)
+            for (int l = 0; l < d; ++l)
+              if (std::abs(Dm[(n - k) * d + n - l] - ((k + l) & 1 ? -1.0 : 1.0) * std::conj(Dm[k * d + l])) > 1e-12) return false;
+        }
+        return true;
+      };
+      if (real && mirrored() && n + 1 <= SPIN_WARPS * SPIN_ROWS && spin_smem(n) <= 227 * 1024) {
+        int4* de;
+        double* dc;
+        if ((rc = dalloc(ctx, &de, ent.size())) || (rc = dalloc(ctx, &dc, sc2.size()))) return rc;
+        CK(cudaMemcpyAsync(de, ent.data(), ent.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->st));
+        CK(cudaMemcpyAsync(dc, sc2.data(), sc2.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->st));
+        CK(cudaStreamSynchronize(ctx->st));     // the host vectors go out of scope
+        t.spin_ent = de; t.spin_c = dc;
+      }
+    }
   }
   return GH_OK;
 }
@@ -840,7 +884,8 @@ int gh_ctx_create(int D, int N, int n_lat, const int* L, const gh_rep_desc* rep,
     stage = std::max<size_t>(stage, (size_t)V * std::max<size_t>(std::max<size_t>((size_t)D * N * N * 2, (size_t)D * ctx->ng), (size_t)ctx->d * 2));
   }
   ctx->nU = u; ctx->nP = p; ctx->nF = f; ctx->nG = g;
-  std::vector<Work> wg, wgp;
+  std::vector<Work> wg, wgp, wspin;
+  int nspin_sites = 0;
   int gw = GEN_WARPS;
   if (ctx->rep == REP_GEN) {
     // one warp per link.  Tensor path: a buffer of N^n complex numbers in shared memory.
@@ -874,6 +919,14 @@ int gh_ctx_create(int D, int N, int n_lat, const int* L, const gh_rep_desc* rep,
       for (int mu = 0; mu < D; ++mu)
         for (int s0 = 0; s0 < ctx->lat_h[l].V; s0 += gw)
           wg.push_back(Work{l, mu, s0, std::min(gw, ctx->lat_h[l].V - s0)});
+    if (N == 2 && ctx->use_sp) {
+      for (int l = 0; l < n_lat; ++l)
+        for (int s0 = 0; s0 < ctx->lat_h[l].V; s0 += ULANE) wspin.push_back(Work{l, -1, s0, std::min(ULANE, ctx->lat_h[l].V - s0)});
+      nspin_sites = (int)wspin.size();
+      for (int l = 0; l < n_lat; ++l)
+        for (int mu = 0; mu < D; ++mu)
+          for (int s0 = 0; s0 < ctx->lat_h[l].V; s0 += ULANE) wspin.push_back(Work{l, mu, s0, std::min(ULANE, ctx->lat_h[l].V - s0)});
+    }
     // irreps inside the adjoint product: the product kernel, one item per 32-site block
     // and direction (taken over the tensor and closed-form paths when available)
     std::string pwhy;
@@ -931,12 +984,13 @@ int gh_ctx_create(int D, int N, int n_lat, const int* L, const gh_rep_desc* rep,
   }
   b.U = U; b.Us = Us; b.P = P; b.phi = phi; b.phis = phis; b.pi = pi; b.psif = psif; b.psib = psib;
   b.nw_links = (int)wl.size(); b.nw_sites = (int)ws.size(); b.nw_gen = (int)wg.size(); b.gen_warps = gw;
+  b.nw_spin = (int)wspin.size(); b.nw_spin_sites = nspin_sites;
   b.nw_gprod = (int)wgp.size(); b.gen_prod = ctx->has_prod ? 1 : 0; b.gen_pair = ctx->has_pair ? 1 : 0;
   b.hist_cap = 1024;
   b.nlat = n_lat; b.D = D; b.N = N; b.d = ctx->d; b.rep = ctx->rep; b.scalar = ctx->scalar; b.st = ctx->st;
   if ((rc = dalloc(ctx, &b.lats, n_lat)) || (rc = dalloc(ctx, &b.w_all, wall.size())) ||
       (rc = dalloc(ctx, &b.w_gen, std::max<size_t>(wg.size(), 1))) ||
-      (rc = dalloc(ctx, &b.w_gprod, std::max<size_t>(wgp.size(), 1))) || (rc = dalloc(ctx, &b.blk_first, blk_first.size())) ||
+      (rc = dalloc(ctx, &b.w_gprod, std::max<size_t>(wgp.size(), 1))) || (rc = dalloc(ctx, &b.w_spin, std::max<size_t>(wspin.size(), 1))) || (rc = dalloc(ctx, &b.blk_first, blk_first.size())) ||
       (rc = dalloc(ctx, &b.partials, (size_t)ws.size() * NRED)) || (rc = dalloc(ctx, &b.res, (size_t)n_lat * 2 * NRES)) ||
       (rc = dalloc(ctx, &b.hist, (size_t)n_lat * b.hist_cap)) || (rc = dalloc(ctx, &b.last, n_lat)) || (rc = dalloc(ctx, &ctx->staging, stage)) ||
       (rc = dalloc(ctx, &ctx->fbuf, (size_t)std::max<long long>(p, 1))) ||
@@ -946,6 +1000,7 @@ int gh_ctx_create(int D, int N, int n_lat, const int* L, const gh_rep_desc* rep,
   CK(cudaMemcpyAsync(b.lats, ctx->lat_h.data(), sizeof(LatDev) * n_lat, cudaMemcpyHostToDevice, ctx->st));
   CK(cudaMemcpyAsync(b.w_all, wall.data(), sizeof(Work) * wall.size(), cudaMemcpyHostToDevice, ctx->st));
   if (!wg.empty()) CK(cudaMemcpyAsync(b.w_gen, wg.data(), sizeof(Work) * wg.size(), cudaMemcpyHostToDevice, ctx->st));
+  if (!wspin.empty()) CK(cudaMemcpyAsync(b.w_spin, wspin.data(), sizeof(Work) * wspin.size(), cudaMemcpyHostToDevice, ctx->st));
   if (!wgp.empty()) CK(cudaMemcpyAsync(b.w_gprod, wgp.data(), sizeof(Work) * wgp.size(), cudaMemcpyHostToDevice, ctx->st));
   CK(cudaMemcpyAsync(b.blk_first, blk_first.data(), sizeof(int) * blk_first.size(), cudaMemcpyHostToDevice, ctx->st));
   if ((rc = rebuild_kick_table(ctx))) { g_err = ctx->err; return rc; }

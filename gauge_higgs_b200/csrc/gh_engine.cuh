@@ -34,6 +34,8 @@ struct Bufs {
   int nw_gen;
   Work* w_gprod;   // general irrep, product of adjoints: items of up to 32 links (one 32-site block)
   int nw_gprod;
+  Work* w_spin;    // k_gen_spin: site items of up to 32 sites, then link items of up to 32 links
+  int nw_spin_sites, nw_spin;
   int gen_prod;    // 1: general-irrep link work through the adjoint product (k_gen_pair, k_gen_sym2 or k_gen_prod)
   int gen_pair;    // 1: general-irrep link work through k_gen_pair (two-slot irreps)
   int gen_warps;   // warps per block of k_gen_links (1..GEN_WARPS, from the tensor size)
@@ -89,6 +91,9 @@ struct Engine : EngineBase {
     if (e == cudaSuccess && b.gen.pq64)
       e = cudaFuncSetAttribute(k_gen_prod<D, N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)gen_prod_smem<N, C>(b.d, b.gen.pnrows));
+    if constexpr (N == 2)
+      if (e == cudaSuccess && b.gen.spin_ent)
+        e = cudaFuncSetAttribute(k_gen_spin<D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spin_smem(b.gen.n));
     if (e == cudaSuccess && b.gen.s2)
       e = cudaFuncSetAttribute(k_gen_sym2<D, N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sym2_smem<N, C>(b.d));
     return e == cudaSuccess ? 0 : -1;
@@ -142,6 +147,14 @@ struct Engine : EngineBase {
         launch(k_gen_prod<D, N, R>, b.nw_gprod, GP_THREADS, gen_prod_smem<N, C>(b.d, b.gen.pnrows), b.st, a);
       }
       return;
+    }
+    if constexpr (N == 2) {
+      if (b.gen.spin_ent && !prod) {                        // {n} in closed form, with the potential's site items
+        const int skip = b.pot == POT_MULTI ? 0 : b.nw_spin_sites;
+        a.work = b.w_spin + skip;
+        launch(k_gen_spin<D, R>, b.nw_spin - skip, SPIN_WARPS * 32, spin_smem(b.gen.n), b.st, a);
+        return;
+      }
     }
     const size_t sm = gen_smem(b);
     launch(k_gen_links<D, N, R>, b.nw_gen, b.gen_warps * 32, sm, b.st, a);

@@ -136,6 +136,8 @@ struct GenTables {                 // general irrep (src/rep/rep_general.hpp), s
   const int* t_ptr;  const int* t_j;  const double2* t_v;    // T^a_R: CSR over (a, row)
   // single-row irreps: D(U) in closed form (host term lists, gh_sympow.h); null: tensor path
   const int* sp_ptr; const double2* sp_c; const unsigned char* sp_e;
+  // SU(2): the same D(U) as real sums over |a|^2, |b|^2 (k_gen_spin); null: not used
+  const int4* spin_ent; const double* spin_c;
   int warp_bytes;                                            // shared memory of one warp
   int px_off;                                                // byte offset of px in a warp's region
   // irreps inside the K-fold adjoint product (host: gh_adjprod.h): the isometric
@@ -942,6 +944,195 @@ __global__ void __launch_bounds__(GEN_WARPS * 32) k_gen_links(const GenArgs a) {
       P[pi_] = (R)((C)P[pi_] - (C)a.eps * F);
     } else {
       a.out[pi_] = (double)F;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// SU(2) irreps {n} in closed form, 32 links per block.  With U's first row (a, b), x = |a|^2
+// and y = |b|^2 the entries of D(U) with k + l <= n are
+//   D_kl = a^(n-k-l) b^(l-k) sum_i s_i x^(m-i) y^i,  m = min(k, l)
+// (conj(b)^(k-l) for l < k; s_i the coefficients of the term list with the signs of U's
+// second row (-conj b, conj a)), and D_(n-k)(n-l) = (-1)^(k+l) conj(D_kl) gives the others:
+// for n = 12 91 entries of 3.3 real terms on average, where the term list has 455 products
+// of four complex powers (k_gen_links).  A lane is a link; the warps split the powers, then
+// the entries, then the rows of psi_f = D phi_y and psi_b = D^dag phi_x; all in FP64
+// whatever the fields.  Work items with mu < 0 are 32 sites for the multi-invariant
+// potential (they come first, being the longest): the upper triangle of M = phi phi^dag, then
+// w = A(M) phi row by row from the nonzeros of A.  Modes and outputs as k_gen_links.
+// Bound: latency of the four phases and shared memory.  SU(2) {12} 8^4 FP64 with the
+// 13-channel potential, cold caches: 43 us against k_gen_links' 111.
+// ---------------------------------------------------------------------------
+constexpr int SPIN_WARPS = 8, SPIN_ROWS = 3;      // rows per warp: d <= 18
+__host__ __device__ constexpr int spin_entries(int n) { return (n + 1) * (n + 2) / 2; }
+__host__ __device__ constexpr int spin_at(int n, int k, int l) { return k * (n + 1) - k * (k - 1) / 2 + l; }
+__host__ __device__ constexpr size_t spin_smem(int n) {
+  return (size_t)32 * (16 * (spin_entries(n) + 2 * (n + 1)) + 8 * 2 * (n / 2 + 1));
+}
+template <int D, typename R>
+__global__ void __launch_bounds__(SPIN_WARPS * 32, 3) k_gen_spin(const GenArgs a) {
+  pdl_enter();
+  typedef typename Cmp<R>::t C;
+  extern __shared__ unsigned char smem_raw[];
+  const Work w = a.work[blockIdx.x];
+  const LatDev& L = a.lats[w.lat];
+  const int n = a.t.n, d = n + 1;
+  const int c = threadIdx.x & 31, q = threadIdx.x >> 5;
+  cx<double>* Dm = reinterpret_cast<cx<double>*>(smem_raw) + c;      // [entries][32]
+  cx<double>* Pa = Dm + 32 * spin_entries(n);                        // [d][32] powers of a, later phi_{x+mu}
+  cx<double>* Pb = Pa + 32 * d;                                      // [d][32] powers of b, later phi_x
+  double* X = reinterpret_cast<double*>(Pb - c + 32 * d) + c;        // [n/2+1][32] powers of x, then of y
+  double* Y = X + 32 * (n / 2 + 1);
+  const int s = w.s0 + (c < w.n ? c : 0);                            // lanes past the lattice's end repeat site s0
+  int x[D];
+  coords<D>(L, s, x);
+  const bool live = c < w.n && below_hi<D>(L, x);
+  const R* phi = (const R*)a.phi;
+  if (w.mu < 0) {                                                    // potential of 32 sites
+    for (int k = q; k < d; k += SPIN_WARPS) Pb[k * 32] = ldc<double>(phi, f_index(L, d, k, s));
+    __syncthreads();
+    for (int e = q; e < d * d; e += SPIN_WARPS) {                    // M_ij, i <= j, at [i][j - i] of a triangle
+      const int i = e / d, j = e - i * d;
+      if (i <= j) Dm[spin_at(n, i, j - i) * 32] = mulc(Pb[i * 32], Pb[j * 32]);
+    }
+    __syncthreads();
+    const double2* __restrict__ av = reinterpret_cast<const double2*>(a.sa.v);
+    const auto m = [&](int ij) {
+      const int i = ij & 0xFF, j = ij >> 8;
+      cx<double> z = Dm[spin_at(n, i < j ? i : j, i < j ? j - i : i - j) * 32];
+      if (i > j) z.im = -z.im;
+      return z;
+    };
+    const auto am = [&](int rq) {
+      cx<double> y = zero<double>();
+      const int e1 = __ldg(a.sa.ptr + rq + 1);
+      int z = __ldg(a.sa.ptr + rq);
+      for (; z + 4 <= e1; z += 4) {                                  // four in flight
+        int ij[4];
+        double2 v[4];
+        cx<double> t[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { ij[k] = __ldg(a.sa.ij + z + k); v[k] = __ldg(av + z + k); }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) t[k] = m(ij[k]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y = cfma(y, mk<double>(v[k].x, v[k].y), t[k]);
+      }
+      for (; z < e1; ++z) {
+        const double2 v = __ldg(av + z);
+        y = cfma(y, mk<double>(v.x, v.y), m(__ldg(a.sa.ij + z)));
+      }
+      return y;
+    };
+    for (int r = q; r < d; r += SPIN_WARPS) {
+      cx<double> acc = zero<double>();
+      for (int k = 0; k < d; ++k) acc = cfma(acc, am(r * d + k), Pb[k * 32]);
+      if (c < w.n) a.wpot[f_index(L, d, r, s)] = make_double2(acc.re, acc.im);
+    }
+    return;
+  }
+  const int mu = w.mu;
+  const bool own = live && in_box<D>(L, x);
+  const int spm = nfwd(L, s, x[mu], mu);
+  cx<double> px[SPIN_ROWS], py[SPIN_ROWS];
+#pragma unroll
+  for (int t = 0; t < SPIN_ROWS; ++t) {
+    const int k = q + SPIN_WARPS * t;
+    if (k < d) { px[t] = ldc<double>(phi, f_index(L, d, k, s)); py[t] = ldc<double>(phi, f_index(L, d, k, spm)); }
+  }
+  if (q < 4) {
+    const cx<double> u = ldc<double>((const R*)a.U, u_index(L, 4, mu, q & 1, s));
+    if (q < 2) {
+      cx<double>* P = q ? Pb : Pa;
+      cx<double> p = mk<double>(1.0, 0.0);
+      for (int k = 0; k < d; ++k) { P[k * 32] = p; p = mul(p, u); }
+    } else {
+      double* P = q == 3 ? Y : X;
+      const double r = norm2(u);
+      double p = 1.0;
+      for (int k = 0; k <= n / 2; ++k) { P[k * 32] = p; p *= r; }
+    }
+  }
+  __syncthreads();
+  for (int e = q; e < spin_entries(n); e += SPIN_WARPS) {
+    const int4 t = __ldg(a.t.spin_ent + e);                          // k, l, first coefficient
+    const int m = t.x < t.y ? t.x : t.y;
+    double r = 0.0;
+#pragma unroll 4
+    for (int i = 0; i <= m; ++i) r = fmad(__ldg(a.t.spin_c + t.z + i) * X[(m - i) * 32], Y[i * 32], r);
+    const cx<double> pb = Pb[(t.y >= t.x ? t.y - t.x : t.x - t.y) * 32];
+    const cx<double> pa = scale(Pa[(n - t.x - t.y) * 32], r);
+    Dm[e * 32] = t.y >= t.x ? mul(pa, pb) : mulc(pa, pb);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < SPIN_ROWS; ++t) {
+    const int k = q + SPIN_WARPS * t;
+    if (k < d) { Pa[k * 32] = py[t]; Pb[k * 32] = px[t]; }
+  }
+  __syncthreads();
+  const auto entry = [&](int k, int l) {
+    if (k + l <= n) return Dm[spin_at(n, k, l) * 32];
+    const cx<double> z = Dm[spin_at(n, n - k, n - l) * 32];
+    return (k + l) & 1 ? mk<double>(-z.re, z.im) : mk<double>(z.re, -z.im);
+  };
+  cx<double> f[SPIN_ROWS];
+#pragma unroll
+  for (int t = 0; t < SPIN_ROWS; ++t) {
+    const int k = q + SPIN_WARPS * t;
+    f[t] = zero<double>();
+    if (k >= d) continue;
+#pragma unroll 4
+    for (int l = 0; l < d; ++l) f[t] = cfma(f[t], entry(k, l), Pa[l * 32]);
+    if (live) stc<double>((R*)a.psif, g_index(L, d, mu, k, s), f[t]);
+  }
+  if (a.mode == 1) return;
+#pragma unroll
+  for (int t = 0; t < SPIN_ROWS; ++t) {
+    const int k = q + SPIN_WARPS * t;
+    if (k >= d) continue;
+    cx<double> z = zero<double>();
+#pragma unroll 4
+    for (int l = 0; l < d; ++l) z = cfma_cj(z, entry(l, k), Pb[l * 32]);
+    if (live) stc<double>((R*)a.psib, g_index(L, d, mu, k, s), z);
+  }
+  __syncthreads();                                                   // phi_{x+mu} and D are read
+#pragma unroll
+  for (int t = 0; t < SPIN_ROWS; ++t)
+    if (q + SPIN_WARPS * t < d) Pa[(q + SPIN_WARPS * t) * 32] = f[t];
+  __syncthreads();
+  // matter force g^a = -2 Im(phi_x^dag T^a_R psi_f): the warps split the rows
+  double F[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int t = 0; t < SPIN_ROWS; ++t) {
+    const int i = q + SPIN_WARPS * t;
+    if (i >= d) continue;
+#pragma unroll
+    for (int g = 0; g < 3; ++g) {
+      cx<double> ti = zero<double>();
+      const int e1 = __ldg(a.t.t_ptr + g * d + i + 1);
+      for (int e = __ldg(a.t.t_ptr + g * d + i); e < e1; ++e) {
+        const double2 tv = __ldg(a.t.t_v + e);
+        ti = cfma(ti, mk<double>(tv.x, tv.y), Pa[__ldg(a.t.t_j + e) * 32]);
+      }
+      F[g] += px[t].re * ti.im - px[t].im * ti.re;
+    }
+  }
+  double* Fs = reinterpret_cast<double*>(smem_raw) + c;
+#pragma unroll
+  for (int g = 0; g < 3; ++g) Fs[(q * 3 + g) * 32] = F[g];
+  __syncthreads();
+  if (q < 3 && own) {
+    double z = 0.0;
+#pragma unroll
+    for (int k = 0; k < SPIN_WARPS; ++k) z += Fs[(k * 3 + q) * 32];
+    const C Fa = -(C)L.kappa * (C(-2) * (C)z);
+    const long long pi_ = p_index(L, 3, mu, q, s);
+    if (a.mode == 0) {
+      R* P = (R*)a.P;
+      P[pi_] = (R)((C)P[pi_] - (C)a.eps * Fa);
+    } else {
+      a.out[pi_] = (double)Fa;
     }
   }
 }
