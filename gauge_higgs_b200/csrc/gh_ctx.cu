@@ -420,28 +420,67 @@ bool kick_linear(const LatDev& L, int D) {
   return ntiles > (L.V + KICK_BLOCK - 1) / KICK_BLOCK;
 }
 
-// Kick items of the lattices in `lats`: link items direction by direction (all
-// tiles of direction 0, then direction 1, ...), then one site item per tile.
-// Direction-major order keeps the blocks resident at one time on distinct sites.
-void kick_items(const gh_ctx* ctx, const std::vector<int>& lats, std::vector<Work>& out, int& nlinks, int& nsites) {
-  std::vector<Work> links, sites, links_mu[4];
+// Kick items of the lattices in `lats`.  Inside a slab (consecutive tiles, lattice after
+// lattice) the link items go direction by direction, so that the blocks resident at one
+// time work on distinct sites.  A launch whose links and momenta fit in L2 is one slab;
+// beyond that each direction's sweep would read every link from HBM again, so slabs are
+// cut at 20 MB of links (adjoint scalar: 12 MB, its site items are long and a slab ends on
+// them): the other directions and the scalar force find them in L2.  Kick in us, one slab
+// and slabs: SU(3) fundamental 32^4 FP32 443 and 368, FP64 879 and 715, 24^4 FP32 146 and
+// 123, FP64 275 and 218, adjoint 24^4 FP64 355 and 331 (403 at 20 MB); below the line slabs
+// lose their ends' idle lanes: SU(2) 24^4 FP64 (117 MB) 66.3 and 69.7, SU(3) 16^4 FP64 (54 MB)
+// 42.8 and 47.
+constexpr size_t KICK_L2_BYTES = 126u << 20, KICK_SLAB_BYTES = 20u << 20, KICK_SLAB_BYTES_ADJ = 12u << 20;
+struct KickTable {
+  std::vector<Work> links, sites, both;
+};
+void kick_items(const gh_ctx* ctx, const std::vector<int>& lats, KickTable& out) {
   const int D = ctx->D;
+  std::vector<Work> mu_items[4], sites;
+  size_t bytes = 0;
+  const auto flush = [&]() {
+    for (int mu = 0; mu < D; ++mu) {
+      out.links.insert(out.links.end(), mu_items[mu].begin(), mu_items[mu].end());
+      out.both.insert(out.both.end(), mu_items[mu].begin(), mu_items[mu].end());
+      mu_items[mu].clear();
+    }
+    if (ctx->scalar) out.both.insert(out.both.end(), sites.begin(), sites.end());
+    out.sites.insert(out.sites.end(), sites.begin(), sites.end());
+    sites.clear();
+    bytes = 0;
+  };
+  const size_t site_bytes = (size_t)D * ctx->N * ctx->N * 2 * ctx->rs;
+  size_t total = 0;
+  for (int l : lats) total += (site_bytes + (size_t)D * ctx->ng * ctx->rs) * ctx->lat_h[l].V;
+  const size_t cut = total <= KICK_L2_BYTES ? total : ctx->rep == REP_ADJ ? KICK_SLAB_BYTES_ADJ : KICK_SLAB_BYTES;
+  const bool split = ctx->rep == REP_GEN && ctx->d >= KICK_SITE_SPLIT_D;
+  out.links.clear();
+  out.sites.clear();
+  out.both.clear();
+  // sites [s0, s0 + n) of a kick_site_gen lattice, and the end of a tile
+  const auto split_sites = [&](int l, int s0, int n) {
+    for (int e = s0 + n; s0 < e; s0 += ULANE) sites.push_back(Work{l, -1, s0, std::min(ULANE, e - s0)});
+  };
+  const auto tile_done = [&](int nsites) {
+    bytes += site_bytes * nsites;
+    if (bytes > cut) flush();
+  };
   for (int l : lats) {
     const LatDev& Ld = ctx->lat_h[l];
-    const bool split = ctx->rep == REP_GEN && ctx->d >= KICK_SITE_SPLIT_D;
-    if (split)
-      for (int s0 = 0; s0 < Ld.V; s0 += ULANE) sites.push_back(Work{l, -1, s0, std::min(ULANE, Ld.V - s0)});
     if (ctx->kick_lin[l]) {
       for (int s0 = 0; s0 < Ld.V; s0 += KICK_BLOCK) {
         const int n = std::min(KICK_BLOCK, Ld.V - s0);
-        for (int mu = 0; mu < D; ++mu) links_mu[mu].push_back(Work{l, mu + KICK_LINEAR, s0, n});
-        if (!split) sites.push_back(Work{l, KICK_LINEAR - 1, s0, n});
+        for (int mu = 0; mu < D; ++mu) mu_items[mu].push_back(Work{l, mu + KICK_LINEAR, s0, n});
+        if (split) split_sites(l, s0, n);
+        else sites.push_back(Work{l, KICK_LINEAR - 1, s0, n});
+        tile_done(n);
       }
       continue;
     }
     int t[4], nt[4];
     long long ntiles = 1;
     for (int mu = 0; mu < 4; ++mu) { t[mu] = 1 << Ld.lt[mu]; nt[mu] = mu < D ? (Ld.L[mu] + t[mu] - 1) / t[mu] : 1; ntiles *= nt[mu]; }
+    const int share = (int)(((Ld.V + ntiles - 1) / ntiles + ULANE - 1) / ULANE * ULANE);   // a tile's share of the 32-site items
     for (long long q = 0; q < ntiles; ++q) {
       long long r = q;
       int s0 = 0, packed = 0;
@@ -451,18 +490,19 @@ void kick_items(const gh_ctx* ctx, const std::vector<int>& lats, std::vector<Wor
         s0 += o * Ld.stride[mu];
         packed |= o << (8 * mu);
       }
-      for (int mu = 0; mu < D; ++mu) links_mu[mu].push_back(Work{l, mu, s0, packed});
+      for (int mu = 0; mu < D; ++mu) mu_items[mu].push_back(Work{l, mu, s0, packed});
       if (!split) sites.push_back(Work{l, -1, s0, packed});
+      else if (q * share < Ld.V) split_sites(l, (int)(q * share), (int)std::min<long long>(share, Ld.V - q * share));
+      tile_done((int)(Ld.V / ntiles));
     }
   }
-  for (int mu = 0; mu < D; ++mu) links.insert(links.end(), links_mu[mu].begin(), links_mu[mu].end());
-  nlinks = (int)links.size();
-  nsites = (int)sites.size();
-  out = links;
-  out.insert(out.end(), sites.begin(), sites.end());
+  flush();
 }
 
-int upload_kick_items(gh_ctx* ctx, const std::vector<Work>& items, int nlinks, int nsites) {
+int upload_kick_items(gh_ctx* ctx, const KickTable& k) {
+  std::vector<Work> items = k.links;
+  items.insert(items.end(), k.sites.begin(), k.sites.end());
+  items.insert(items.end(), k.both.begin(), k.both.end());
   if (items.size() > ctx->wk_cap) {
     if (ctx->wk_dev) cudaFree(ctx->wk_dev);
     ctx->wk_dev = nullptr;
@@ -472,8 +512,8 @@ int upload_kick_items(gh_ctx* ctx, const std::vector<Work>& items, int nlinks, i
   }
   CK(cudaMemcpyAsync(ctx->wk_dev, items.data(), sizeof(Work) * items.size(), cudaMemcpyHostToDevice, ctx->st));
   ctx->b.w_kick = ctx->wk_dev;
-  ctx->b.nwk_links = nlinks;
-  ctx->b.nwk_sites = nsites;
+  ctx->b.nwk_links = (int)k.links.size();
+  ctx->b.nwk_sites = (int)k.sites.size();
   ctx->b.kick_lin = 0;
   for (const Work& w : items) ctx->b.kick_lin |= w.mu >= KICK_LINEAR - 1;
   return GH_OK;
@@ -491,11 +531,10 @@ int rebuild_kick_table(gh_ctx* ctx) {
   if (rc) return rc;
   std::vector<int> all(ctx->nlat);
   for (int l = 0; l < ctx->nlat; ++l) all[l] = l;
-  std::vector<Work> items;
-  int nl, ns;
-  kick_items(ctx, all, items, nl, ns);
+  KickTable items;
+  kick_items(ctx, all, items);
   invalidate_graph(ctx);
-  return upload_kick_items(ctx, items, nl, ns);
+  return upload_kick_items(ctx, items);
 }
 
 // Lift and projection tables of k_gen_sym2; false where the irrep has no symmetric-tensor
@@ -1409,10 +1448,9 @@ int gh_autotune(gh_ctx* ctx, int reps, double* best_ms) {
       for (int l : lats) { std::memcpy(ctx->lat_h[l].lt, lt, sizeof(lt)); ctx->kick_lin[l] = lin; }
       int rc = push_tiles(ctx);
       if (rc) return rc;
-      std::vector<Work> items;
-      int nl, ns;
-      kick_items(ctx, lats, items, nl, ns);
-      if ((rc = upload_kick_items(ctx, items, nl, ns))) return rc;
+      KickTable items;
+      kick_items(ctx, lats, items);
+      if ((rc = upload_kick_items(ctx, items))) return rc;
       ctx->eng->kick(ctx->b, 0.0, M_UPDATE, F_GAUGE | F_MATTER, nullptr, true, true);
       CK(cudaEventRecord(e0, ctx->st));
       for (int r = 0; r < reps; ++r) ctx->eng->kick(ctx->b, 0.0, M_UPDATE, F_GAUGE | F_MATTER, nullptr, true, true);

@@ -40,7 +40,7 @@ struct Bufs {
   int gen_pair;    // 1: general-irrep link work through k_gen_pair (two-slot irreps)
   int gen_warps;   // warps per block of k_gen_links (1..GEN_WARPS, from the tensor size)
   int* blk_first;  // [nlat+1] first site item of each lattice (relative to the site items)
-  Work* w_kick;    // kick items: link items then site items, over 4-D tiles (LatDev::lt) or consecutive sites
+  Work* w_kick;    // kick items over 4-D tiles (LatDev::lt) or consecutive sites: links, sites, then both slab by slab
   int kick_lin;    // 1: some items are consecutive sites
   int nwk_links, nwk_sites;
   double* partials;
@@ -106,7 +106,7 @@ struct Engine : EngineBase {
     a.sa = sizeof(R) == sizeof(double) ? b.sa64 : b.sa32;
     a.wpot = b.wpot;
     const bool do_sites = sites && b.scalar;
-    const int first = links ? 0 : b.nwk_links;
+    const int first = links && do_sites ? b.nwk_links + b.nwk_sites : links ? 0 : b.nwk_links;
     const int count = (links ? b.nwk_links : 0) + (do_sites ? b.nwk_sites : 0);
     if (count == 0) return;
     a.work = b.w_kick + first;
