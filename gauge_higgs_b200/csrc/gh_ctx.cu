@@ -244,10 +244,9 @@ void enq_trajectory(gh_ctx* ctx) {
   Bufs& b = ctx->b;
   InitArgs ia{};
   ia.what = 1; ia.pure = ctx->scalar ? 0 : 1; ia.real = ctx->real; ia.d = ctx->d; ia.vec = b.pi;
+  ia.Us = b.Us; ia.phi = b.phi; ia.phis = b.phis;   // saved beside the draws, which leave memory idle
   ctx->eng->init(b, ia, true, ctx->scalar != 0);
   if (b.frozen) ctx->eng->sphere(b, 0);   // tangent-space momenta (src/hmc/gauge_higgs_hmc.hpp:172)
-  cudaMemcpyAsync(b.Us, b.U, (size_t)ctx->nU * 2 * ctx->rs, cudaMemcpyDeviceToDevice, ctx->st);
-  if (ctx->scalar) cudaMemcpyAsync(b.phis, b.phi, (size_t)ctx->nF * 2 * ctx->rs, cudaMemcpyDeviceToDevice, ctx->st);
   enq_measure(ctx, 0);
   enq_md(ctx);
   if (ctx->prec == GH_PREC_FP64) ctx->eng->reunit(b);

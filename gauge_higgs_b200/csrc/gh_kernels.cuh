@@ -2158,7 +2158,14 @@ struct InitArgs {
   int d;
   double sigma;
   unsigned long long stream;
+  void* Us;           // what == 1: also save U and phi here (the trajectory's reject copy); null: no
+  const void* phi;
+  void* phis;
 };
+// component c of `nc` of every site or link, saved at the same place
+template <typename V> __device__ __forceinline__ void save_components(const void* from, void* to, long long first, int nc) {
+  for (int c = 0; c < nc; ++c) reinterpret_cast<V*>(to)[first + c * ULANE] = reinterpret_cast<const V*>(from)[first + c * ULANE];
+}
 // Gaussian draw for a field stored as R: the correctly rounded draw for FP64
 // fields, the CUDA-libm draw for FP32 fields (identical after rounding to FP32
 // but for ~1e-8 of draws).
@@ -2174,6 +2181,10 @@ __global__ void __launch_bounds__(KBLOCK) k_init(const InitArgs a) {
   if ((int)threadIdx.x >= w.n) return;
   const LatDev L = a.lats[w.lat];
   const int s = w.s0 + threadIdx.x;
+  if (a.what == 1 && a.Us) {
+    if (w.mu >= 0) save_components<typename V2<R>::t>(a.U, a.Us, u_index(L, N * N, w.mu, 0, s), N * N);
+    else save_components<typename V2<R>::t>(a.phi, a.phis, f_index(L, a.d, 0, s), a.d);
+  }
   if (!active_site(L, s)) return;                 // halo sites come from the neighbours
   const long long gs = global_site(L, s);         // the RNG key's site
   constexpr int ng = N * N - 1;
