@@ -402,20 +402,38 @@ template <typename T> GH_HD Mat<3, T> expi3(const Mat<3, T>& H) {
   const Mat<3, T> Q2 = herm_sq3(Q);   // H (and Q) Hermitian: built from real algebra coefficients
   const T c1 = T(0.5) * (Q2.e[0].re + Q2.e[4].re + Q2.e[8].re);
   const T c0 = det_herm3(Q);
-  // (a, b, g): the coefficients of Q^n / n! in (I, Q, Q^2), advanced two terms per trip
-  // (i^n = i, -1 for n = 4k+1, 4k+2 and -i, 1 for n = 4k+3, 4k+4)
-  T a = 1, b = 0, g = 0;
-  T f0r = 1, f0i = 0, f1r = 0, f1i = 0, f2r = 0, f2i = 0;
+  T f0r, f0i, f1r, f1i, f2r, f2i;
+  if (!(nrm2 > T(0.04))) {
+    // ||Q||_F <= 1/5 (an MD step has about 1/16): the terms to n = 11 with the powers written
+    // out in c0 and c1 (Q^5 = c0 c1 + c1^2 Q + c0 Q^2, ...); the first one left out is below
+    // 0.2^12 / 12! = 9e-18.  A third of the loop's operations, and no test per pair of terms:
+    // SU(3) 16^4 trajectories 1249 -> 1222 us (FP32-MD), 1981 -> 1959 (FP64)
+    const T r3 = T(1.0 / 6), r4 = T(1.0 / 24), r5 = T(1.0 / 120), r6 = T(1.0 / 720), r7 = T(1.0 / 5040), r8 = T(1.0 / 40320),
+            r9 = T(1.0 / 362880), r10 = T(1.0 / 3628800), r11 = T(1.0 / 39916800);
+    const T q = c0 * c0, c3 = c1 * c1 * c1;
+    f0r = fmad(-q, fmad(c1, fmad(T(3) * r10, c1, T(-2) * r8), r6), T(1));
+    f0i = c0 * fmad(c1, fmad(c1, fmad(c1, fmad(-r11, c1, r9), -r7), r5), fmad(q, fmad(T(-3) * r11, c1, r9), -r3));
+    f1r = c0 * fmad(c1, fmad(T(3) * r8, c1, T(-2) * r6), fmad(-r10, fmad(T(4), c3, q), r4));
+    f1i = fmad(c1, fmad(c1, fmad(c1, fmad(c1, fmad(-r11, c1, r9), -r7), r5), -r3),
+               fmad(q, fmad(c1, fmad(T(-6) * r11, c1, T(3) * r9), -r7), T(1)));
+    f2r = fmad(c1, fmad(c1, fmad(c1, fmad(-r10, c1, r8), -r6), r4), fmad(q, fmad(T(-3) * r10, c1, r8), T(-0.5)));
+    f2i = c0 * fmad(c1, fmad(T(3) * r9, c1, T(-2) * r7), fmad(-r11, fmad(T(4), c3, q), r5));
+  } else {
+    f0r = 1, f0i = 0, f1r = 0, f1i = 0, f2r = 0, f2i = 0;
+    // (a, b, g): the coefficients of Q^n / n! in (I, Q, Q^2), advanced two terms per trip
+    // (i^n = i, -1 for n = 4k+1, 4k+2 and -i, 1 for n = 4k+3, 4k+4)
+    T a = 1, b = 0, g = 0;
 #pragma unroll
-  for (int n = 1; n < 40; n += 2) {
-    const T sg = (n & 2) ? T(-1) : T(1);
-    T r = (T)inv_int(n);
-    T an = c0 * g * r, bn = fmad(c1, g, a) * r, gn = b * r;
-    f0i = fmad(sg, an, f0i); f1i = fmad(sg, bn, f1i); f2i = fmad(sg, gn, f2i);
-    r = (T)inv_int(n + 1);
-    a = c0 * gn * r; b = fmad(c1, gn, an) * r; g = bn * r;
-    f0r = fmad(-sg, a, f0r); f1r = fmad(-sg, b, f1r); f2r = fmad(-sg, g, f2r);
-    if (fabs(a) + fabs(b) + fabs(g) < T(ExpTol<T>::v)) break;
+    for (int n = 1; n < 40; n += 2) {
+      const T sg = (n & 2) ? T(-1) : T(1);
+      T r = (T)inv_int(n);
+      T an = c0 * g * r, bn = fmad(c1, g, a) * r, gn = b * r;
+      f0i = fmad(sg, an, f0i); f1i = fmad(sg, bn, f1i); f2i = fmad(sg, gn, f2i);
+      r = (T)inv_int(n + 1);
+      a = c0 * gn * r; b = fmad(c1, gn, an) * r; g = bn * r;
+      f0r = fmad(-sg, a, f0r); f1r = fmad(-sg, b, f1r); f2r = fmad(-sg, g, f2r);
+      if (fabs(a) + fabs(b) + fabs(g) < T(ExpTol<T>::v)) break;
+    }
   }
   Mat<3, T> E;
 #pragma unroll
