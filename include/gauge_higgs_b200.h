@@ -345,9 +345,9 @@ int gh_rep_product_matrix(int N, const gh_rep_desc* rep, const double* U, double
  * links before using it.
  * Irreps of n = K N boxes inside the K-fold adjoint product (K = 1, 2; SU(3): the
  * octet {2,1}, the 27-plet {4,2}, the 10bar {3,3}) take GH_PATH_PRODUCT instead, when
- * the context finds and checks the intertwiner (gh_rep_product_matrix): a lift by a
- * fixed A x d matrix shared by 32 links per block, the adjoint matrix of each link
- * applied K times, a projection -- the reference's tensor matrix to rounding.  The
+ * the context finds and checks the intertwiner (gh_rep_product_matrix): the octet as
+ * U Phi U^dag on N x N matrices, the 27-plet on symmetric tensors Phi^{ij}_{kl}, others
+ * with the adjoint matrix of each link -- the reference's tensor matrix to rounding.  The
  * multi-invariant potential's per-site term is computed on the tensor / closed-form
  * path, so contexts with that potential use it for their link work.
  * Two-slot irreps outside that product (n = 2: SU(3) sextet {2}, antitriplet {1,1})
