@@ -197,7 +197,9 @@ struct Engine : EngineBase {
     const int count = (links ? b.nw_links : 0) + (sites ? b.nw_sites : 0);
     if (count == 0) return;
     a.work = b.w_all + first;
-    launch(k_init<N, R>, count, KBLOCK, 0, b.st, a);
+    const bool draws = a.what >= 1 && a.what <= 3;
+    if (draws && (count < INIT_SPLIT_BLOCKS || (sites && a.d >= INIT_SPLIT_D))) launch(k_init<N, R, true>, 4 * count, KBLOCK, 0, b.st, a);
+    else launch(k_init<N, R, false>, count, KBLOCK, 0, b.st, a);
   }
   void restore(const Bufs& b) override {
     RestoreArgs a;

@@ -2162,9 +2162,10 @@ struct InitArgs {
   const void* phi;
   void* phis;
 };
-// component c of `nc` of every site or link, saved at the same place
-template <typename V> __device__ __forceinline__ void save_components(const void* from, void* to, long long first, int nc) {
-  for (int c = 0; c < nc; ++c) reinterpret_cast<V*>(to)[first + c * ULANE] = reinterpret_cast<const V*>(from)[first + c * ULANE];
+// components c0, c0 + cs, ... of the `nc` of a site or link, saved at the same place
+template <typename V>
+__device__ __forceinline__ void save_components(const void* from, void* to, long long first, int nc, int c0, int cs) {
+  for (int c = c0; c < nc; c += cs) reinterpret_cast<V*>(to)[first + c * ULANE] = reinterpret_cast<const V*>(from)[first + c * ULANE];
 }
 // Gaussian draw for a field stored as R: the correctly rounded draw for FP64
 // fields, the CUDA-libm draw for FP32 fields (identical after rounding to FP32
@@ -2173,17 +2174,31 @@ template <typename R> __device__ __forceinline__ double gauss_r(uint64_t seed, u
   return sizeof(R) == sizeof(double) ? ghrng::gauss(seed, k) : ghrng::gauss_md(seed, k);
 }
 
-template <int N, typename R>
+// SPLIT (Gaussian draws): four blocks per item, a lane per site and the components of a
+// link or vector split over the warps.  A thread that draws all of them in turn is a chain
+// of 8 (links) to 2 d draws, which a launch of few blocks waits for; beyond
+// INIT_SPLIT_BLOCKS items the chains of other threads hide it, and the key's common part
+// would be hashed by four threads.  Refresh in us, whole and split: 6^4 SU(2) FP64 9.0 and 7.2,
+// SU(3) 9^3 x 12 adjoint 22.3 and 14.9, 12^4 sextet 40.9 and 33.0, 27-plet 75.8 and 44.9, SU(2)
+// {12} 8^4 37.1 and 15.5.
+constexpr int INIT_SPLIT_BLOCKS = 148 * 6;   // one wave of whole items at 80 registers
+constexpr int INIT_SPLIT_D = 9;              // from this many vector components on in any launch
+template <int N, typename R, bool SPLIT>
 __global__ void __launch_bounds__(KBLOCK) k_init(const InitArgs a) {
   pdl_enter();
   typedef typename Cmp<R>::t C;
-  const Work w = a.work[blockIdx.x];
-  if ((int)threadIdx.x >= w.n) return;
+  static_assert(KBLOCK == 4 * ULANE, "a split item is four blocks of 32 sites");
+  const Work w = a.work[SPLIT ? blockIdx.x >> 2 : blockIdx.x];
+  const int i = SPLIT ? (int)(blockIdx.x & 3) * ULANE + (int)(threadIdx.x & (ULANE - 1)) : (int)threadIdx.x;
+  if (i >= w.n) return;
   const LatDev L = a.lats[w.lat];
-  const int s = w.s0 + threadIdx.x;
+  const int s = w.s0 + i;
+  // this thread's components: c0, c0 + cs, ...
+  const int c0 = SPLIT ? (int)threadIdx.x / ULANE : 0;
+  constexpr int cs = SPLIT ? 4 : 1;
   if (a.what == 1 && a.Us) {
-    if (w.mu >= 0) save_components<typename V2<R>::t>(a.U, a.Us, u_index(L, N * N, w.mu, 0, s), N * N);
-    else save_components<typename V2<R>::t>(a.phi, a.phis, f_index(L, a.d, 0, s), a.d);
+    if (w.mu >= 0) save_components<typename V2<R>::t>(a.U, a.Us, u_index(L, N * N, w.mu, 0, s), N * N, c0, cs);
+    else save_components<typename V2<R>::t>(a.phi, a.phis, f_index(L, a.d, 0, s), a.d, c0, cs);
   }
   if (!active_site(L, s)) return;                 // halo sites come from the neighbours
   const long long gs = global_site(L, s);         // the RNG key's site
@@ -2206,7 +2221,10 @@ __global__ void __launch_bounds__(KBLOCK) k_init(const InitArgs a) {
       R* P = (R*)a.P;
       const long long pb = p_index(L, ng, mu, 0, s);
 #pragma unroll
-      for (int g = 0; g < ng; ++g) P[pb + g * ULANE] = (R)gauss_r<R>(L.seed, ghrng::key(st, gs, mu, g));
+      for (int q = 0; q < (ng + cs - 1) / cs; ++q) {
+        const int g = c0 + q * cs;
+        if (g < ng) P[pb + g * ULANE] = (R)gauss_r<R>(L.seed, ghrng::key(st, gs, mu, g));
+      }
     }
     return;
   }
@@ -2216,7 +2234,7 @@ __global__ void __launch_bounds__(KBLOCK) k_init(const InitArgs a) {
     const unsigned long long st = (a.what == 1) ? ghrng::key(0xD4, L.traj) : a.stream;
     const double sg = (a.what == 1) ? 1.0 : a.sigma;
     R* vec = (R*)a.vec;
-    for (int k = 0; k < a.d; ++k) {
+    for (int k = c0; k < a.d; k += cs) {
       const double re = sg * gauss_r<R>(L.seed, ghrng::key(st, gs, 2 * k));
       const double im = a.real ? 0.0 : sg * gauss_r<R>(L.seed, ghrng::key(st, gs, 2 * k + 1));
       stc<double>(vec, f_index(L, a.d, k, s), mk<double>(re, im));
