@@ -25,6 +25,16 @@ inline void launch(void (*kernel)(A), unsigned grid, unsigned block, size_t smem
   cudaLaunchKernelEx(&cfg, kernel, args);
 }
 
+// The limit on a kernel's dynamic shared memory belongs to the kernel, not to a context: every
+// context sets the same one, all that a block may have beside the kernel's static part, so
+// none lowers it under another that lives.  Each launch still passes its own size.
+template <typename A>
+inline cudaError_t allow_smem(void (*kernel)(A)) {
+  cudaFuncAttributes fa;
+  const cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes);
+}
+
 struct Bufs {
   void *U, *Us, *P, *phi, *phis, *pi, *psif, *psib;
   LatDev* lats;
@@ -87,15 +97,11 @@ struct Engine : EngineBase {
   }
   int prepare(const Bufs& b) override {
     if (REP != REP_GEN) return 0;
-    cudaError_t e = cudaFuncSetAttribute(k_gen_links<D, N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gen_smem(b));
-    if (e == cudaSuccess && b.gen.pq64)
-      e = cudaFuncSetAttribute(k_gen_prod<D, N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)gen_prod_smem<N, C>(b.d, b.gen.pnrows));
+    cudaError_t e = allow_smem(k_gen_links<D, N, R>);
+    if (e == cudaSuccess && b.gen.pq64) e = allow_smem(k_gen_prod<D, N, R>);
     if constexpr (N == 2)
-      if (e == cudaSuccess && b.gen.spin_ent)
-        e = cudaFuncSetAttribute(k_gen_spin<D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spin_smem(b.gen.n));
-    if (e == cudaSuccess && b.gen.s2)
-      e = cudaFuncSetAttribute(k_gen_sym2<D, N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sym2_smem<N, C>(b.d));
+      if (e == cudaSuccess && b.gen.spin_ent) e = allow_smem(k_gen_spin<D, R>);
+    if (e == cudaSuccess && b.gen.s2) e = allow_smem(k_gen_sym2<D, N, R>);
     return e == cudaSuccess ? 0 : -1;
   }
   void kick(const Bufs& b, double eps, int mode, int flags, double* out, bool links, bool sites) override {
