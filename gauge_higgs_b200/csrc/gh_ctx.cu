@@ -275,13 +275,21 @@ int run_traj(gh_ctx* ctx) {
                                    "layer (global dH and accept), not by the device Metropolis");
   if (ctx->use_graph) {
     if (!ctx->gexec) {
+      cudaGetLastError();   // what an earlier call left and reported is not this capture's
       CK(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
       enq_trajectory(ctx);
       cudaGraph_t g = nullptr;
       cudaError_t e = cudaStreamEndCapture(ctx->st, &g);
       if (e != cudaSuccess) { cudaGetLastError(); return fail(ctx, GH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e)); }
       ctx->graph = g;
-      CK(cudaGraphInstantiate(&ctx->gexec, g, 0));
+      // a launch that failed is not in the graph: it must not be replayed without that kernel
+      int rc = launch_check(ctx, "trajectory");
+      if (!rc && (e = cudaGraphInstantiate(&ctx->gexec, g, 0)) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->gexec = nullptr;
+        rc = fail(ctx, GH_ERR_CUDA, std::string("graph instantiation: ") + cudaGetErrorString(e));
+      }
+      if (rc) { invalidate_graph(ctx); return rc; }
     }
     CK(cudaGraphLaunch(ctx->gexec, ctx->st));
   } else {
