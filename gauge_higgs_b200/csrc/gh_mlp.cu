@@ -336,6 +336,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(TW * 32) k_steps(co
 // at the barriers between them.  The sums run in the same order as there.
 // ---------------------------------------------------------------------------
 constexpr int RT = 512;      // threads
+constexpr int RES_SMEM = 227 * 1024;   // all that a block may have
 struct ResLayout {           // offsets in floats
   int Bp, RS, RH;            // batch rounded up to 32; row strides: floats RS (odd), halves RH (odd words)
   int dup;                   // the output layer is computed by every block
@@ -676,7 +677,7 @@ bool res_layout(const Net& n, int maxB, ResLayout& L) {
     L.m2[l] = take(nc * (nin + 1));
   }
   L.total = (int)std::min<long>(at, 1 << 28);
-  return at * sizeof(float) <= 227 * 1024;
+  return at * sizeof(float) <= RES_SMEM;
 }
 
 __global__ void k_adam(float* p, const float* g, float* m1, float* m2, long n, float lr, float b1, float b2, float eps,
@@ -766,7 +767,9 @@ int run_steps(Net* n, int mode, const std::vector<StepInfo>& steps, const std::v
   ResArgs ra;
   if (mode != FORWARD && res_layout(*n, maxB, ra.L)) {
     void (*const k)(ResArgs) = ra.L.Bp == 32 ? k_steps_resident<32> : ra.L.Bp == 64 ? k_steps_resident<64> : k_steps_resident<0>;
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, ra.L.total * (int)sizeof(float));
+    // the limit belongs to the kernel: the same one from every network, or a call of a narrower
+    // network in another thread could lower it between this and the launch
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM);
     ra.s = t;
     if (!e) k<<<n->M * CL, RT, ra.L.total * sizeof(float)>>>(ra);
     e = e ? e : cudaGetLastError();
