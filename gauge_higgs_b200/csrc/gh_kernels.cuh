@@ -1349,8 +1349,9 @@ __global__ void __launch_bounds__(GP_THREADS) k_gen_prod(const GenArgs a) {
 // Split: one block per 32 links of a direction, a warp per column (then per row), a lane
 // per link: shared memory is read without conflicts and every table entry is uniform.
 // Bound: latency, on 18 warps per SM (FP64 pipe 29% busy, shared memory 45%; about 7,000
-// multiply-adds per link).  3 blocks per SM (312 bytes spilled) beat 2 without spills by 4%,
-// FP32 5 beat 4 by 2%.
+// multiply-adds per link).  3 blocks per SM (284 bytes spilled) beat 2 without spills by 4%.
+// FP32 fields, whose force is summed in double too: kick and drift at 12^4 with 3 / 4 / 5 blocks
+// 98.9 / 93.6 / 103.1 us (83.1 with the force in FP32, 350 with k_gen_prod).
 // ---------------------------------------------------------------------------
 constexpr int S2_NNZ = 64, S2_DMAX = 36, S2_PAIRS = 36;   // largest tables the kernel takes
 struct Sym2Tab {
@@ -1364,14 +1365,15 @@ template <int N> struct Sym2 {
   static constexpr int NS = N * (N + 1) / 2, THREADS = 32 * NS;
   __host__ __device__ static constexpr int pair(int i, int j) { return i <= j ? i * N - i * (i - 1) / 2 + j - i : j * N - j * (j - 1) / 2 + i - j; }
 };
-// 32-lane complex rows of one phi buffer; the force's NS x ng real partial sums take its place later
-template <int N> __host__ __device__ constexpr int sym2_rows(int d) {
-  const int need = (Sym2<N>::NS * (N * N - 1) + 1) / 2;
+// 32-lane complex rows of the phi_{x+mu} buffer, which the force's NS x ng partial sums (double)
+// take over once it is lifted
+template <int N, typename C> __host__ __device__ constexpr int sym2_rows(int d) {
+  constexpr int need = Sym2<N>::NS * (N * N - 1) * (int)sizeof(double) / (int)sizeof(cx<C>) + 1;
   return d > need ? d : need;
 }
-// phi_x, phi_{x+mu} (then the force's partial sums), the tensor
+// phi_x, phi_{x+mu} (then the partial sums), the tensor
 template <int N, typename C> __host__ __device__ constexpr size_t sym2_smem(int d) {
-  return (size_t)(2 * sym2_rows<N>(d) + Sym2<N>::NS * Sym2<N>::NS) * 32 * 2 * sizeof(C);
+  return (size_t)(d + sym2_rows<N, C>(d) + Sym2<N>::NS * Sym2<N>::NS) * 32 * sizeof(cx<C>);
 }
 // O = V M V^T for a symmetric M (pairs i <= j); V_ij = U_ij, transposed (TR) and / or conjugated (CJ)
 template <int N, bool TR, bool CJ, typename C>
@@ -1400,21 +1402,22 @@ __device__ __forceinline__ void sym2_rotate(const Mat<N, C>& U, const cx<C>* M, 
     }
   }
 }
-// F += or -= w Im Tr T^a (P X^dag)  (or its transpose), P and X symmetric
+// F += or -= w Im Tr T^a (P X^dag)  (or its transpose), P and X symmetric; in double whatever
+// the fields, since the rows' and the columns' terms cancel in part
 template <int N, bool MINUS_T, typename C>
-__device__ __forceinline__ void sym2_force(const cx<C>* P, const cx<C>* X, C w, C* F) {
-  Mat<N, C> R;
+__device__ __forceinline__ void sym2_force(const cx<C>* P, const cx<C>* X, double w, double* F) {
+  Mat<N, double> R;
 #pragma unroll
   for (int i = 0; i < N; ++i)
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      cx<C> s = zero<C>();
+      cx<double> s = zero<double>();
 #pragma unroll
-      for (int k = 0; k < N; ++k) s = cfma_cj(s, X[Sym2<N>::pair(k, j)], P[Sym2<N>::pair(i, k)]);
+      for (int k = 0; k < N; ++k) s = cfma_cj(s, cvt<double>(X[Sym2<N>::pair(k, j)]), cvt<double>(P[Sym2<N>::pair(i, k)]));
       R.e[MINUS_T ? j * N + i : i * N + j] = s;
     }
-  C f[N * N - 1];
-  im_tr_proj<N, C>(R, f);
+  double f[N * N - 1];
+  im_tr_proj<N, double>(R, f);
 #pragma unroll
   for (int g = 0; g < N * N - 1; ++g) F[g] = fmad(MINUS_T ? -w : w, f[g], F[g]);
 }
@@ -1429,7 +1432,7 @@ template <typename C> __device__ __forceinline__ C s2_proj(const Sym2Tab& t, int
 }
 
 template <int D, int N, typename R>
-__global__ void __launch_bounds__(Sym2<N>::THREADS, sizeof(R) == 8 ? 3 : 5) k_gen_sym2(const __grid_constant__ Sym2Args a) {
+__global__ void __launch_bounds__(Sym2<N>::THREADS, sizeof(R) == 8 ? 3 : 4) k_gen_sym2(const __grid_constant__ Sym2Args a) {
   pdl_enter();
   typedef typename Cmp<R>::t C;
   constexpr int NS = Sym2<N>::NS, ng = N * N - 1;
@@ -1439,9 +1442,9 @@ __global__ void __launch_bounds__(Sym2<N>::THREADS, sizeof(R) == 8 ? 3 : 5) k_ge
   const int d = a.g.t.d;
   const int c = threadIdx.x & 31, q = threadIdx.x >> 5;   // lane: link; warp: column J, then row I
   cx<C>* Px = reinterpret_cast<cx<C>*>(smem_raw) + c;     // [d][32] phi_x
-  cx<C>* Py = Px + 32 * sym2_rows<N>(d);                  // [d][32] phi_{x+mu}
-  cx<C>* X = Py + 32 * sym2_rows<N>(d);                   // [NS][NS][32]
-  C* Fs = reinterpret_cast<C*>(Py - c) + c;               // [NS][ng][32], once phi_{x+mu} is lifted
+  cx<C>* Py = Px + 32 * d;                                // [d][32] phi_{x+mu}
+  cx<C>* X = Py + 32 * sym2_rows<N, C>(d);                // [NS][NS][32]
+  double* Fs = reinterpret_cast<double*>(Py - c) + c;     // [NS][ng][32], once phi_{x+mu} is lifted
   const int mu = w.mu;
   const int s = w.s0 + (c < w.n ? c : 0);                 // lanes past the lattice's end compute on site s0
   int x[D];
@@ -1485,7 +1488,7 @@ __global__ void __launch_bounds__(Sym2<N>::THREADS, sizeof(R) == 8 ? 3 : 5) k_ge
   bool diag = false;
 #pragma unroll
   for (int i = 0; i < N; ++i) diag = diag || q == Sym2<N>::pair(i, i);
-  const C k4 = C(4) * (C)L.kappa * (diag ? C(1) : C(2));
+  const double k4 = 4.0 * L.kappa * (diag ? 1.0 : 2.0);
   __syncthreads();
   cx<C> M[NS], O[NS];
   lift(Py, q, NS, M);                                     // psi_f = D phi_{x+mu}: columns, U
@@ -1498,10 +1501,10 @@ __global__ void __launch_bounds__(Sym2<N>::THREADS, sizeof(R) == 8 ? 3 : 5) k_ge
   sym2_rotate<N, false, true, C>(U, M, O);
 #pragma unroll
   for (int i = 0; i < NS; ++i) X[(q * NS + i) * 32] = O[i];
-  C F[ng];
+  double F[ng];
   if (a.g.mode != 1) {
 #pragma unroll
-    for (int g = 0; g < ng; ++g) F[g] = C(0);
+    for (int g = 0; g < ng; ++g) F[g] = 0.0;
     lift(Px, q * NS, 1, M);
     sym2_force<N, true, C>(O, M, k4, F);
   }
@@ -1519,7 +1522,7 @@ __global__ void __launch_bounds__(Sym2<N>::THREADS, sizeof(R) == 8 ? 3 : 5) k_ge
     for (int g = q; g < ng; g += NS) {
       double f = 0.0;
 #pragma unroll
-      for (int j = 0; j < NS; ++j) f += (double)Fs[(j * ng + g) * 32];
+      for (int j = 0; j < NS; ++j) f += Fs[(j * ng + g) * 32];
       const long long pi_ = p_index(L, ng, mu, g, s);
       if (a.g.mode == 0) {
         R* P = (R*)a.g.P;
