@@ -718,7 +718,7 @@ int build_general(gh_ctx* ctx, const gh_rep_desc* r) {
         }
         return true;
       };
-      if (real && mirrored() && n + 1 <= SPIN_WARPS * SPIN_ROWS && spin_smem(n) <= 227 * 1024) {
+      if (real && mirrored() && spin_fits(n)) {
         int4* de;
         double* dc;
         if ((rc = dalloc(ctx, &de, ent.size())) || (rc = dalloc(ctx, &dc, sc2.size()))) return rc;

@@ -971,6 +971,11 @@ __host__ __device__ constexpr int spin_at(int n, int k, int l) { return k * (n +
 __host__ __device__ constexpr size_t spin_smem(int n) {
   return (size_t)32 * (16 * (spin_entries(n) + 2 * (n + 1)) + 8 * 2 * (n / 2 + 1));
 }
+// what the kernel can take: its rows, a block's shared memory, and room over D's entries for the
+// force's partial sums (3 per warp), which must not reach the vectors behind them: n >= 4
+__host__ __device__ constexpr bool spin_fits(int n) {
+  return n + 1 <= SPIN_WARPS * SPIN_ROWS && spin_smem(n) <= 227 * 1024 && 16 * spin_entries(n) >= 8 * 3 * SPIN_WARPS;
+}
 template <int D, typename R>
 __global__ void __launch_bounds__(SPIN_WARPS * 32, 3) k_gen_spin(const GenArgs a) {
   pdl_enter();
