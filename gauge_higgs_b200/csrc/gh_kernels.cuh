@@ -615,12 +615,15 @@ __device__ __forceinline__ void kick_link_dispatch(const KickArgs& a, const LatD
   }
 }
 
-// Occupancy: resident kick blocks per SM.  FP32: 7 (72 registers, 40 bytes spilled by the
-// fundamental), the adjoint 5 (its commutator terms spill 432 bytes at 72 registers against
-// 28 at 96); FP64: 4 (128 registers, 64 bytes spilled), the adjoint 3 (it spills 1.3 KB at
-// 128 registers).  General irreps, whose link part is the gauge force alone, gain from the
-// same: trajectories at SU(3) 12^4, FP32 5 and 7 blocks, octet 1366 and 1275 us, sextet 1225
-// and 1185; FP64 3 and 4, 27-plet 6650 and 6425.  Measured at
+// Occupancy: resident kick blocks per SM.  FP32: 7 (72 registers; the fundamental spills 40
+// bytes with tiles, 84 with consecutive sites), the adjoint 5 (its commutator terms spill 432
+// bytes at 72 registers against 28 at 96); FP64: 4 (128 registers, 88 and 8 bytes spilled), the
+// adjoint 3 (it spills 1.3 KB at 128 registers).  General irreps, whose link part is the gauge
+// force alone, gain from the same: trajectories at SU(3) 12^4, FP32 5 and 7 blocks, octet 1366
+// and 1275 us, sextet 1225 and 1185; FP64 3 and 4, 27-plet 6650 and 6425.  Pure gauge does not
+// (nothing else runs between its kicks but the drift) and keeps 5 and 3: kick at 6^4, 12^4, 16^4
+// with 5 / 7 blocks FP32 4.6 / 5.4, 10.3 / 12.1, 20.9 / 20.8 us, with 3 / 4 blocks FP64 5.2 / 6.1,
+// 14.3 / 15.1, 33.2 / 35.0.  Measured at
 // SU(3) 16^4 (fundamental): the kick alone runs the same at FP32 5 and 7 blocks (24.5
 // us) and at FP64 3 and 4 (40.7 / 40.9 us), while the trajectory with the higher
 // occupancy is 1.4% (FP32) and 1.7% (FP64) faster -- the next launch's blocks find room
@@ -647,11 +650,11 @@ __device__ __forceinline__ void kick_link_dispatch(const KickArgs& a, const LatD
 #define GH_KICK_MINB_F64_FUND 4
 #endif
 template <int N, typename R, int REP> struct KickMinBlocks {
-  static constexpr int b = N == 2 ? GH_KICK_MINB_F32_SU2 : REP != REP_ADJ ? GH_KICK_MINB_F32_FUND : GH_KICK_MINB_F32;
+  static constexpr int b = N == 2 ? GH_KICK_MINB_F32_SU2 : REP == REP_FUND || REP == REP_GEN ? GH_KICK_MINB_F32_FUND : GH_KICK_MINB_F32;
   static constexpr int v = b * 128 / KICK_BLOCK;
 };
 template <int N, int REP> struct KickMinBlocks<N, double, REP> {
-  static constexpr int b = N == 2 ? GH_KICK_MINB_F64_SU2 : REP != REP_ADJ ? GH_KICK_MINB_F64_FUND : GH_KICK_MINB_F64;
+  static constexpr int b = N == 2 ? GH_KICK_MINB_F64_SU2 : REP == REP_FUND || REP == REP_GEN ? GH_KICK_MINB_F64_FUND : GH_KICK_MINB_F64;
   static constexpr int v = b * 128 / KICK_BLOCK > 0 ? b * 128 / KICK_BLOCK : 1;
 };
 
