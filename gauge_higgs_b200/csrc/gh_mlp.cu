@@ -35,7 +35,7 @@ struct Net {
   int cap = 0;                // batch capacity of the activation buffers
   float* z[MAXL] = {};        // [M][width[l+1]][cap] pre-activations (FP32)
   __nv_bfloat16* a[MAXL] = {};  // [M][width[l+1]][cap] activations (BF16), last layer unused
-  float* out = nullptr;       // [M][n_out][cap]
+  float* out = nullptr;       // [M][cap][n_out]
   float* gz[MAXL] = {};       // [M][width[l+1]][cap] gradients w.r.t. pre-activations
   float* loss = nullptr;      // [loss_cap][M]
   int loss_cap = 0;
@@ -45,6 +45,8 @@ struct Net {
   long idx_cap = 0;
   StepInfo* steps = nullptr;
   long step_cap = 0;
+  float *xs = nullptr, *ys = nullptr;   // a step's samples in its order (layer by layer)
+  long xs_cap = 0, ys_cap = 0;
   std::string err;
 };
 
@@ -58,9 +60,8 @@ __device__ __forceinline__ float dsilu(float z) { const float s = 1.f / (1.f + _
 // One kernel runs whole optimiser steps (or one gradient, or a forward pass): a cluster of
 // CL blocks per network, which meets at the cluster's hardware barrier between layers.  A
 // step is seven dependent layers of a few hundred kFLOP, so its time is latency: as
-// separate launches (13 per step and two blocking copies of the minibatch, each thread
-// walking its rows or columns of the weights alone in global memory) a step of 5 networks
-// 4-128-128-128-3 at batch 32 took 333 us; here 43 us.
+// separate launches (each thread walking its rows or columns of the weights alone in global
+// memory) a step of 5 networks 4-128-128-128-3 at batch 32 takes 267 us; here 43 us.
 // Each layer is one tile product out[row][col] = init[col] + sum_k W(col, k) X(row, k):
 //   forward   row = sample, col = neuron j, k = input i:  z = b + W a
 //   backward  row = sample, col = input i,  k = neuron j: gz' = (W^T gz) silu'(z')
@@ -235,7 +236,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(TW * 32) k_steps(co
             t.z[l][o] = v;
             t.a[l][o] = __float2bfloat16(silu(v));
           } else {
-            t.out[o] = v;
+            t.out[(m * cap + first + b) * nout + j] = v;
             if (t.mode != FORWARD) {
               const float d = v - t.y[sample(b) * nout + j];
               t.gz[l][o] = 2.f * d / (float)(B * nout);
@@ -255,7 +256,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(TW * 32) k_steps(co
       if (threadIdx.x < 256) {
         float s = 0.f;
         for (int e = threadIdx.x; e < B * nout; e += 256) {
-          const float d = t.out[(m * nout + e % nout) * cap + e / nout] - t.y[sample(e / nout) * nout + e % nout];
+          const float d = t.out[m * cap * nout + e] - t.y[sample(e / nout) * nout + e % nout];
           s += d * d;
         }
         sh[threadIdx.x] = s;
@@ -686,6 +687,115 @@ __global__ void k_adam(float* p, const float* g, float* m1, float* m2, long n, f
     adam_update(p + e, m1 + e, m2 + e, g[e], lr, b1, b2, eps, c1, c2);
 }
 
+// ---------------------------------------------------------------------------
+// The same arithmetic with one launch per layer and product, over the whole GPU, for the calls
+// whose work fills it: a cluster has 8 of its 148 SMs.  Which form a call takes: cluster_us and
+// layers_us.  Activations and gradients lie [sample][neuron] here.  Sums in the order of k_steps.
+// Bound: one thread's chain of multiply-adds in small calls (a neuron's weights, or the batch),
+// the shared and L1 loads beside each multiply-add in large ones.
+// ---------------------------------------------------------------------------
+constexpr int BT = 16;       // samples per block (forward and input gradient)
+struct LayerArgs {
+  int B, nin, nout;
+  long cap, P;                 // samples per network in the buffers; parameters per network
+  const float *w, *bias;       // network 0's
+  const float* x;              // layer 0: the step's samples, else null
+  const __nv_bfloat16* in;     // other layers: activations
+};
+
+// a step's samples and targets in its order
+__global__ void k_gather(const float* x, const float* y, const int* idx, int B, int nin, int nout, float* xs, float* ys) {
+  const int row = nin + nout;
+  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < (long)B * row; e += (long)gridDim.x * blockDim.x) {
+    const int b = (int)(e / row), k = (int)(e - (long)b * row);
+    if (k < nin) xs[(long)b * nin + k] = x[(long)idx[b] * nin + k];
+    else ys[(long)b * nout + k - nin] = y[(long)idx[b] * nout + k - nin];
+  }
+}
+
+// z = b + W a, and the next layer's activations (a null: none); a thread per neuron
+__global__ void __launch_bounds__(1024) k_dense_fwd(const LayerArgs t, float* z, __nv_bfloat16* a) {
+  extern __shared__ float s_in[];   // [BT][nin]
+  const int tiles = (t.B + BT - 1) / BT, m = blockIdx.x / tiles, b0 = (blockIdx.x - m * tiles) * BT, j = threadIdx.x;
+  const int nin = t.nin, rows = min(BT, t.B - b0);
+  const __nv_bfloat16* in = t.in + (m * t.cap + b0) * nin;
+  for (int e = threadIdx.x; e < BT * nin; e += blockDim.x)
+    s_in[e] = e >= rows * nin ? 0.f : t.x ? t.x[(long)b0 * nin + e] : __bfloat162float(in[e]);
+  __syncthreads();
+  if (j >= t.nout) return;
+  const float* w = t.w + m * t.P + (long)j * nin;
+  float acc[BT];
+#pragma unroll
+  for (int bb = 0; bb < BT; ++bb) acc[bb] = t.bias[m * t.P + j];
+  for (int i = 0; i < nin; ++i) {
+    const float wi = w[i];
+#pragma unroll
+    for (int bb = 0; bb < BT; ++bb) acc[bb] = fmaf(wi, s_in[bb * nin + i], acc[bb]);
+  }
+#pragma unroll
+  for (int bb = 0; bb < BT; ++bb) {
+    if (bb >= rows) break;
+    const long o = (m * t.cap + b0 + bb) * t.nout + j;
+    z[o] = acc[bb];
+    if (a) a[o] = __float2bfloat16(silu(acc[bb]));
+  }
+}
+
+// output gradient 2 (out - y) / (B n_out), and the loss where its slot is not null
+__global__ void __launch_bounds__(256) k_mse(const LayerArgs t, const float* out, const float* y, float* gz, float* loss) {
+  const int m = blockIdx.x, n = t.B * t.nout;
+  out += m * t.cap * t.nout;
+  gz += m * t.cap * t.nout;
+  float s = 0.f;
+  for (int e = threadIdx.x; e < n; e += 256) {
+    const float d = out[e] - y[e];
+    s += d * d;
+    gz[e] = 2.f * d / (float)n;
+  }
+  __shared__ float sh[256];
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0 && loss) loss[m] = sh[0] / (float)n;
+}
+
+// dW[j][i] = sum_b gz[b][j] in[b][i], db[j] = sum_b gz[b][j]; a block per neuron, threads over i
+template <bool FIRST>
+__global__ void __launch_bounds__(128) k_dense_wgrad(const LayerArgs t, const float* gz, float* g, long woff, long boff) {
+  const int m = blockIdx.x, j = blockIdx.y, nin = t.nin, nout = t.nout, B = t.B;
+  gz += m * t.cap * nout + j;
+  g += m * t.P;
+  for (int i = threadIdx.x; i <= nin; i += blockDim.x) {
+    const int ic = min(i, nin - 1);
+    const float* x = t.x + ic;
+    const __nv_bfloat16* in = t.in + m * t.cap * nin + ic;
+    float s = 0.f;
+    for (int b = 0; b < B; ++b) {              // the bias's thread walks along with its warp
+      const float v = FIRST ? x[(long)b * nin] : __bfloat162float(in[(long)b * nin]);
+      s = fmaf(gz[(long)b * nout], i == nin ? 1.f : v, s);
+    }
+    g[i == nin ? boff + j : woff + (long)j * nin + i] = s;
+  }
+}
+
+// gradient through the layer and the SiLU before it; a thread per input
+__global__ void __launch_bounds__(1024) k_dense_bgrad(const LayerArgs t, const float* gz, const float* zprev, float* gprev) {
+  const int tiles = (t.B + BT - 1) / BT, m = blockIdx.x / tiles, b0 = (blockIdx.x - m * tiles) * BT, i = threadIdx.x;
+  const int nin = t.nin, nout = t.nout;
+  if (i >= nin) return;
+  const float* w = t.w + m * t.P + i;
+  for (int b = b0; b < min(t.B, b0 + BT); ++b) {
+    const float* gb = gz + (m * t.cap + b) * nout;
+    float s = 0.f;
+    for (int j = 0; j < nout; ++j) s = fmaf(w[(long)j * nin], gb[j], s);
+    const long o = (m * t.cap + b) * nin + i;
+    gprev[o] = s * dsilu(zprev[o]);
+  }
+}
+
 int ensure_cap(Net* n, int B) {
   if (B <= n->cap) return GH_OK;
   auto fr = [](void* q) { if (q) cudaFree(q); };
@@ -738,17 +848,105 @@ int upload_samples(Net* n, const float* x, const float* y, long ns) {
   return GH_OK;
 }
 
+// Which form a call takes: the two are bit for bit the same, and which is faster turns on every
+// size, so both times are estimated (us per step or pass) from what each form does.
+//   Clusters: networks (forward: 64-sample pieces of them) in waves of 14, and in each product of
+//   a wave its passes over a block's columns, and the multiply-adds of a lane.
+//   Layers: per product the longer of one thread's chain and the multiply-adds of all networks at
+//   the rate that the kernel reaches with the GPU full.
+// The constants are fitted (rms 9 to 20%) to trainings and predictions of 2025 combinations: 1 to
+// 5 hidden layers of 16 to 512, 1 to 48 networks, batches of 32 to 8192.  A step in us, layers /
+// clusters: 5 networks 4-128-128-128-3, batch 32 267 / 41 (resident), 2048 1310 / 1140; one
+// 4-256-256-256-3, batch 512 950 / 960, 2048 1830 / 3700; 48 of 4-16-16-16-3, batch 64 124 / 95,
+// 2048 670 / 1440.
+struct ClusterCost { double call, product, pass, term; };
+constexpr ClusterCost STEPS_COST{16.2, 1.15, 0.955, 4.45e-4}, RESIDENT_COST{13.8, 0.98, 0.648, 2.43e-4},
+    FORWARD_COST{44.9, 0.81, 0.383, 4.68e-4};
+constexpr int CLUSTERS_AT_ONCE = 14;   // clusters of 8 SMs that find room in the GPU's parts
+double cluster_us(const Net& n, int mode, int B, const ClusterCost& c) {
+  const auto up = [](long a, long b) { return (double)((a + b - 1) / b); };
+  const auto product = [&](int rows, int cols, int terms) {
+    return c.product + up(cols, TW) * (up(rows, RG) * up(terms, KC) * c.pass + up(rows, 32) * 32 * terms * c.term);
+  };
+  const int rows = mode == FORWARD ? std::min(B, 64) : B;
+  double t = 0;
+  for (int l = 0; l < n.nl; ++l) {
+    const int nin = n.width[l], nout = n.width[l + 1], ci = (nin + CL - 1) / CL, co = (nout + CL - 1) / CL;
+    t += product(rows, co, nin);
+    if (mode != FORWARD) t += product(nin, co, B) + (l ? product(B, ci, nout) : 0.0);
+  }
+  return c.call + t * up(mode == FORWARD ? (long)n.M * ((B + 63) / 64) : n.M, CLUSTERS_AT_ONCE);
+}
+double layers_us(const Net& n, int mode, int B) {
+  double t = mode == FORWARD ? 23.6 : 47.5;
+  for (int l = 0; l < n.nl; ++l) {
+    const double nin = n.width[l], nout = n.width[l + 1], fma = (double)n.M * B * nin * nout;
+    if (mode == FORWARD) { t += 6.8 + std::max(0.149 * nin, 3.38e-7 * fma); continue; }
+    t += std::max(0.073 * nin, 9.0e-7 * fma) + std::max(0.06 * B * std::ceil((nin + 1) / 128), 2.73e-7 * fma);
+    if (l) t += std::max(0.99 * nout, 2.47e-7 * fma);
+  }
+  return t;
+}
+
+// One step (or forward pass) layer by layer.
+cudaError_t run_layers(const StepArgs& t, const StepInfo& si, float* xs, float* ys) {
+  LayerArgs q{};
+  const float *x = t.x, *y = t.y;
+  if (t.idx) {
+    const int n0 = t.width[0], no = t.width[t.nl];
+    k_gather<<<std::min(((long)si.B * (n0 + no) + 255) / 256, 1024L), 256>>>(x, y, t.idx + si.s0, si.B, n0, no, xs, ys);
+    x = xs;
+    y = ys;
+  }
+  q.B = si.B; q.cap = t.cap; q.P = t.P;
+  const auto layer = [&](int l) {
+    q.nin = t.width[l]; q.nout = t.width[l + 1];
+    q.w = t.p + t.woff[l]; q.bias = t.p + t.boff[l];
+    q.x = l ? nullptr : x;
+    q.in = l ? t.a[l - 1] : nullptr;
+  };
+  const unsigned tiles = (unsigned)t.M * ((si.B + BT - 1) / BT);
+  const auto threads = [](int n) { return (n + 31) / 32 * 32; };
+  const int nl = t.nl;
+  cudaError_t e = cudaFuncSetAttribute(k_dense_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, BT * 1024 * (int)sizeof(float));
+  if (e) return e;
+  for (int l = 0; l < nl; ++l) {
+    layer(l);
+    k_dense_fwd<<<tiles, threads(std::max(q.nin, q.nout)), sizeof(float) * BT * q.nin>>>(q, l == nl - 1 ? t.out : t.z[l], l == nl - 1 ? nullptr : t.a[l]);
+  }
+  if (t.mode != FORWARD) {
+    k_mse<<<t.M, 256>>>(q, t.out, y, t.gz[nl - 1], si.slot >= 0 ? t.loss + (long)si.slot * t.M : nullptr);
+    for (int l = nl - 1; l >= 0; --l) {
+      layer(l);
+      const dim3 grid(t.M, q.nout);
+      if (l) k_dense_wgrad<false><<<grid, 128>>>(q, t.gz[l], t.g, t.woff[l], t.boff[l]);
+      else k_dense_wgrad<true><<<grid, 128>>>(q, t.gz[l], t.g, t.woff[l], t.boff[l]);
+      if (l) k_dense_bgrad<<<tiles, threads(q.nin)>>>(q, t.gz[l], t.z[l - 1], t.gz[l - 1]);
+    }
+    if (t.mode == TRAIN) k_adam<<<296, 256>>>(t.p, t.g, t.m1, t.m2, t.P * t.M, t.lr, t.b1, t.b2, t.eps, si.c1, si.c2);
+  }
+  return cudaGetLastError();
+}
+
 // Runs `steps` (one for FORWARD and GRADIENT) over the uploaded samples; order: sample
 // index of every row of the steps, null for the order they lie in.
 int run_steps(Net* n, int mode, const std::vector<StepInfo>& steps, const std::vector<int>* order, int slots, float lr) {
+  int maxB = 0;
+  for (const StepInfo& q : steps) maxB = std::max(maxB, q.B);
+  ResArgs ra;
+  const bool resident = mode != FORWARD && res_layout(*n, maxB, ra.L);
+  // clusters only where their estimate is clearly the lower
+  const bool layers = layers_us(*n, mode, maxB) < 1.1 * cluster_us(*n, mode, maxB, mode == FORWARD ? FORWARD_COST : resident ? RESIDENT_COST : STEPS_COST);
   long lc = (long)n->loss_cap * n->M;
-  cudaError_t e = grow(&n->steps, &n->step_cap, (long)steps.size());
-  if (!e && order) e = grow(&n->idx, &n->idx_cap, (long)order->size());
-  if (!e) e = grow(&n->loss, &lc, (long)std::max(slots, 1) * n->M);
+  cudaError_t e = cudaSuccess;
+  if (order) e = grow(&n->idx, &n->idx_cap, (long)order->size());
+  if (!e && slots) e = grow(&n->loss, &lc, (long)slots * n->M);
   n->loss_cap = (int)(lc / n->M);
-  if (!e) e = cudaMemcpy(n->steps, steps.data(), sizeof(StepInfo) * steps.size(), cudaMemcpyHostToDevice);
   if (!e && order) e = cudaMemcpy(n->idx, order->data(), sizeof(int) * order->size(), cudaMemcpyHostToDevice);
-  if (!e) e = cudaFuncSetAttribute(k_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STEP_SMEM);
+  if (!e && layers && order) e = grow(&n->xs, &n->xs_cap, (long)maxB * n->width[0]);
+  if (!e && layers && order) e = grow(&n->ys, &n->ys_cap, (long)maxB * n->width[n->nl]);
+  if (!e && !layers) e = grow(&n->steps, &n->step_cap, (long)steps.size());
+  if (!e && !layers) e = cudaMemcpy(n->steps, steps.data(), sizeof(StepInfo) * steps.size(), cudaMemcpyHostToDevice);
   if (e) { cudaGetLastError(); return mfail(n, GH_ERR_CUDA, std::string("MLP steps: ") + cudaGetErrorString(e)); }
   StepArgs t{};
   t.nl = n->nl; t.M = n->M; t.mode = mode; t.nsteps = (int)steps.size();
@@ -762,24 +960,22 @@ int run_steps(Net* n, int mode, const std::vector<StepInfo>& steps, const std::v
   t.x = n->xd; t.y = n->yd; t.idx = order ? n->idx : nullptr;
   t.out = n->out; t.loss = n->loss; t.steps = n->steps;
   t.lr = lr; t.b1 = 0.9f; t.b2 = 0.999f; t.eps = 1e-8f;
-  int maxB = 0;
-  for (const StepInfo& q : steps) maxB = std::max(maxB, q.B);
-  ResArgs ra;
-  if (mode != FORWARD && res_layout(*n, maxB, ra.L)) {
+  if (layers) {
+    for (size_t k = 0; k < steps.size() && !e; ++k) e = run_layers(t, steps[k], n->xs, n->ys);
+  } else if (resident) {
     void (*const k)(ResArgs) = ra.L.Bp == 32 ? k_steps_resident<32> : ra.L.Bp == 64 ? k_steps_resident<64> : k_steps_resident<0>;
     // the limit belongs to the kernel: the same one from every network, or a call of a narrower
     // network in another thread could lower it between this and the launch
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM);
     ra.s = t;
     if (!e) k<<<n->M * CL, RT, ra.L.total * sizeof(float)>>>(ra);
-    e = e ? e : cudaGetLastError();
-    if (e) return mfail(n, GH_ERR_CUDA, std::string("MLP kernel: ") + cudaGetErrorString(e));
-    return GH_OK;
+  } else {
+    t.rows = 64;                                // forward rows are independent: clusters of 64 samples
+    const int gy = mode == FORWARD ? (steps[0].B + t.rows - 1) / t.rows : 1;
+    e = cudaFuncSetAttribute(k_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STEP_SMEM);
+    if (!e) k_steps<<<dim3(n->M * CL, gy), TW * 32, STEP_SMEM>>>(t);
   }
-  t.rows = 64;                                  // forward rows are independent: clusters of 64 samples
-  const int gy = mode == FORWARD ? (steps[0].B + t.rows - 1) / t.rows : 1;
-  k_steps<<<dim3(n->M * CL, gy), TW * 32, STEP_SMEM>>>(t);
-  e = cudaGetLastError();
+  e = e ? e : cudaGetLastError();
   if (e) return mfail(n, GH_ERR_CUDA, std::string("MLP kernel: ") + cudaGetErrorString(e));
   return GH_OK;
 }
@@ -834,7 +1030,7 @@ int gh_mlp_create(int n_members, const int* widths, int n_layers, uint64_t seed,
 int gh_mlp_destroy(gh_mlp* n) {
   if (!n) return GH_OK;
   cudaDeviceSynchronize();
-  void* ps[] = {n->p, n->g, n->m1, n->m2, n->loss, n->xd, n->yd, n->idx, n->steps, n->out};
+  void* ps[] = {n->p, n->g, n->m1, n->m2, n->loss, n->xd, n->yd, n->idx, n->steps, n->xs, n->ys, n->out};
   for (void* q : ps) if (q) cudaFree(q);
   for (int l = 0; l < n->nl; ++l) {
     if (n->z[l]) cudaFree(n->z[l]);
@@ -949,7 +1145,7 @@ int gh_mlp_predict(gh_mlp* n, const float* x, int B, float* per_member, float* m
     for (int k = 0; k < nout; ++k) {
       double s = 0.0, s2 = 0.0;
       for (int m = 0; m < n->M; ++m) {
-        const double v = o[((size_t)m * nout + k) * n->cap + b];
+        const double v = o[((size_t)m * n->cap + b) * nout + k];
         if (per_member) per_member[((size_t)m * B + b) * nout + k] = (float)v;
         s += v;
         s2 += v * v;
