@@ -420,7 +420,13 @@ void default_tile(const int* L, int D, int* lt) {
 // its coordinates.  Measured, whole trajectories with the tiles and with consecutive
 // sites: SU(3) adjoint FP64 9^3 x 12 (1080 blocks, 345 linear) 1597 -> 1096 us, sextet
 // FP64 12^4 (1440, 810) 2239 -> 1984 us, SU(2) FP32 ladder of 6, 8, 10, 12 (10760, 5680)
-// 2250 -> 1760 us.
+// 2250 -> 1760 us; subdomains with their halo, kick and drift: SU(3) FP64 16^4 in 18 x 16^3 92
+// -> 63 us, in 18^4 126 -> 88, FP32 8^4 in 10^4 17.2 -> 14.1.  Where it gains least: launches of a
+// few dozen blocks, whose time hangs on the instruction cache, go either way by shape (SU(3)
+// FP32 kick and drift 6^4 8.8 -> 10.1 us, 6^3 x 7 a quarter less; SU(2) gains a tenth
+// throughout); with fields of 50 to 100 MB their placement in L2 moves one and the same launch
+// by 15%, so both forms were timed at fourteen placements: adjoint FP64 16 x 17 x 16^2 92 to 113 us
+// with tiles, 80 to 111 with consecutive sites.
 bool kick_linear(const LatDev& L, int D) {
   long long ntiles = 1;
   for (int mu = 0; mu < D; ++mu) ntiles *= (L.L[mu] + (1 << L.lt[mu]) - 1) >> L.lt[mu];

@@ -477,7 +477,8 @@ class Ensemble:
         return np.frombuffer(recs, dtype=dt, count=ntraj * self.n_lat).copy().reshape(ntraj, self.n_lat)
 
     def autotune(self, reps=3):
-        """Pick the kick tile of every group of equal-extent lattices by timing."""
+        """Pick the kick blocks (tiles, or consecutive sites where the default tile idles
+        threads) of every group of equal-extent lattices by timing."""
         ms = C.c_double()
         self.ctx("gh_autotune", int(reps), C.byref(ms))
         return ms.value
@@ -487,6 +488,7 @@ class Ensemble:
         self.ctx("gh_set_tile", lat, t)
 
     def get_tile(self, lat=0):
+        """The tile shape; a lattice on consecutive-site blocks does not use it until set_tile."""
         t = (C.c_int * 4)()
         self.ctx("gh_get_tile", lat, t)
         return list(t)[:self.D]

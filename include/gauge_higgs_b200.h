@@ -193,12 +193,17 @@ int gh_read_records(gh_ctx* ctx, int ntraj, gh_traj_record* records);
  * FP32 roundings, which the next upload reproduces). */
 int gh_trajectory_host(gh_ctx* ctx, double* U, double* phi, gh_traj_record* rec);
 /* ---- kick tiles and the autotuner ----
- * The kick kernel gives each 128-thread block a 4-D tile of sites (power-of-two
- * extents per direction); the tile decides how many neighbour links a block
- * reuses from L1.  gh_autotune times every admissible tile on each group of
- * equal-extent lattices (reps zero-step kicks each) and keeps the fastest;
- * best_ms (may be NULL): sum over groups of the best kick time.  Results do not
- * depend on the tile (every link and site is computed the same way). */
+ * A kick block has 128 threads and takes a 4-D tile of sites (power-of-two extents per
+ * direction), or, where the default tile would leave threads idle (extents that it does
+ * not divide), 128 consecutive sites.  The choice decides how many neighbour links a
+ * block reuses from L1.  gh_autotune times every admissible tile, and consecutive sites
+ * where the default took them, on each group of equal-extent lattices (reps zero-step
+ * kicks each) and keeps the fastest; best_ms (may be NULL): sum over groups of the best
+ * kick time.  gh_set_tile sets tiles, also in place of consecutive sites; gh_get_tile
+ * returns the tile shape, which blocks of consecutive sites do not use: after
+ * gh_set_tile(gh_get_tile()) such a lattice runs with tiles until gh_autotune decides
+ * again.  Results do not depend on any of it (every link and site is computed the same
+ * way). */
 int gh_autotune(gh_ctx* ctx, int reps, double* best_ms);
 int gh_set_tile(gh_ctx* ctx, int lat, const int* tile);
 int gh_get_tile(gh_ctx* ctx, int lat, int* tile);
