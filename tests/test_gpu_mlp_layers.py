@@ -56,3 +56,20 @@ def test_wide_network_at_a_large_batch():
     assert abs(loss[0] - lo) < 1e-3 * lo
     assert np.linalg.norm(g[0] - go) < 2e-2 * np.linalg.norm(go)
     net.close()
+
+
+@pytest.mark.parametrize("widths", [(4, 250, 3), (4, 33, 16, 3)])
+def test_members_with_small_batches(widths):
+    """96 members layer by layer, two with everything in their clusters' shared memory."""
+    from gauge_higgs_b200.mlp import MLPEnsemble
+    x, y = data(62, widths[0], widths[-1])
+    out = []
+    for members in (96, 2):
+        net = MLPEnsemble(widths, members=members, seed=5)
+        g, loss = net.grad(x, y)
+        net.adam_step(1e-3)
+        last = net.train(x, y, epochs=3, batch=33, lr=1e-3)
+        out.append([a[:2] for a in (g, loss, last, net.params())])
+        net.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
